@@ -17,6 +17,7 @@ import math
 import random
 
 import torch
+import torch.utils.checkpoint
 
 from pippy_b200.models.gpt2 import GPT2Config, gpt2_loss
 from pippy_b200.models.llama import Llama, LlamaConfig, causal_lm_loss
@@ -261,3 +262,173 @@ def tolerance(case):
     if kind == "adamw":
         return {"rel": 1e-4, "max": 0.01}
     return {"rel": 0.01, "max": 0.4}
+
+
+# ------------------------------------------------------------------------------------------------
+# the same results in 64 bits, from plain torch operations
+# ------------------------------------------------------------------------------------------------
+def _again(fn, *args):
+    """``fn(*args)`` without keeping its intermediates for the backward."""
+    return torch.utils.checkpoint.checkpoint(fn, *args, use_reentrant=False)
+
+
+def _attend64(q, k, v):  # [heads of one key group, S, D], [S, D], [S, D]
+    mask = torch.ones(k.shape[0], k.shape[0], dtype=torch.bool, device=k.device).triu(1)
+    return (q @ k.T / math.sqrt(k.shape[1])).masked_fill(mask, float("-inf")).softmax(-1) @ v
+
+
+def _attention64(qkv, S, heads, kv_heads, hd, rotary, theta=10000.0):
+    q, k, v = (t.view(-1, S, t.shape[1] // hd, hd).transpose(1, 2)
+               for t in qkv.split([heads * hd, kv_heads * hd, kv_heads * hd], dim=1))
+    if rotary:
+        inv = theta ** (-torch.arange(0, hd, 2, dtype=torch.float64, device=qkv.device) / hd)
+        ang = torch.outer(torch.arange(S, dtype=torch.float64, device=qkv.device), inv)
+        c, s = ang.cos(), ang.sin()
+
+        def rotate(x):
+            a, b = x[..., : hd // 2], x[..., hd // 2:]
+            return torch.cat([a * c - b * s, b * c + a * s], dim=-1)
+
+        q, k = rotate(q), rotate(k)
+    rep = heads // kv_heads
+    out = [torch.cat([_again(_attend64, q[b, j * rep:(j + 1) * rep], k[b, j], v[b, j]) for j in range(kv_heads)])
+           for b in range(q.shape[0])]
+    return torch.stack(out).transpose(1, 2).reshape(-1, heads * hd)
+
+
+def _llama64(c, w, ids):
+    """Logits of one batch; ``w`` holds the weights by name."""
+    hd = c["dim"] // c["heads"]
+
+    def norm(x, g):
+        return x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + 1e-5) * g
+
+    def layer(x, i):
+        n = f"layers.{i}."
+        qkv = norm(x, w[n + "attention_norm.weight"]) @ w[n + "attention.wqkv.weight"].T
+        x = x + _attention64(qkv, ids.shape[1], c["heads"], c["kv_heads"], hd, True) @ w[n + "attention.wo.weight"].T
+        g, u = (norm(x, w[n + "ffn_norm.weight"]) @ w[n + "feed_forward.w_gate_up.weight"].T).chunk(2, dim=-1)
+        return x + (torch.nn.functional.silu(g) * u) @ w[n + "feed_forward.w_down.weight"].T
+
+    x = w["tok_embeddings.weight"][ids.reshape(-1)]
+    for i in range(c["layers"]):
+        x = _again(layer, x, i)
+    return norm(x, w["norm.weight"]) @ w["output.weight"].T
+
+
+def _gpt264(c, w, ids):
+    def norm(x, n):
+        return torch.nn.functional.layer_norm(x, x.shape[-1:], w[n + ".weight"], w[n + ".bias"], 1e-5)
+
+    def lin(x, n):
+        return x @ w[n + ".weight"].T + w[n + ".bias"]
+
+    def layer(x, i):
+        n = f"h.{i}."
+        qkv = lin(norm(x, n + "ln_1"), n + "attn_c_attn")
+        x = x + lin(_attention64(qkv, ids.shape[1], c["heads"], c["heads"], 64, False), n + "attn_c_proj")
+        h = torch.nn.functional.gelu(lin(norm(x, n + "ln_2"), n + "mlp_c_fc"), approximate="tanh")
+        return x + lin(h, n + "mlp_c_proj")
+
+    x = w["wte.weight"][ids.reshape(-1)] + w["wte.positions"][: ids.shape[1]].repeat(ids.shape[0], 1)
+    for i in range(c["layers"]):
+        x = _again(layer, x, i)
+    return (norm(x, "ln_f") @ w["wte.weight"].T)[:, : c["vocab"]]
+
+
+def _adamw64(w, grad, lr, betas, eps, decay):
+    """(weights, m, v) after the first step."""
+    m, v = (1 - betas[0]) * grad, (1 - betas[1]) * grad ** 2
+    return w * (1 - lr * decay) - lr * grad / (grad.abs() + eps), m, v
+
+
+def _step64(c, state):
+    pipe = state["pipe"]
+    opt = pipe.optimizer
+    params = {n: p for s in pipe.stages for n, p in s.submod.named_parameters()}
+    w = {n: p.detach().double().requires_grad_() for n, p in params.items()}
+    loss = 0.0
+    for b in range(c["batch"]):  # every sequence has the same number of targets: the mean of means is the mean
+        logits = (_llama64 if c["kind"] == "llama" else _gpt264)(c, w, state["ids"][b:b + 1])
+        part = torch.nn.functional.cross_entropy(logits, state["target"][b]) / c["batch"]
+        part.backward()
+        loss = loss + part.detach()
+    names = {id(p): n for n, p in params.items()}
+    weights, ms, vs = [], [], []
+    for g in opt.groups:
+        flat = g.data.double()
+        grad = torch.zeros_like(flat)
+        for p, o in zip(g.params, g.offsets):
+            grad[o:o + p.numel()] = w[names[id(p)]].grad.reshape(-1)
+        new = _adamw64(flat, grad, opt.lr, opt.betas, opt.eps, opt.weight_decay)
+        for out, x in zip((weights, ms, vs), new):
+            out.append(x)
+    return dict(loss=loss, weights=weights, m=ms, v=vs)
+
+
+def _moe64(c, state):
+    layer, x, dy = state["layer"], state["x"].detach().double(), state["dy"].double()
+    E, k, f = c["experts"], c["top_k"], c["ffn"]
+    router = layer.router.detach().double()
+    x.requires_grad_()
+    router.requires_grad_()
+    logits = (x @ router.T)[:, :E]
+    probs = logits.softmax(-1)
+    # the choice is made on logits of the layer's own 16 bits: a near tie is not a matter of precision
+    chosen = torch.sort(logits.detach().to(BF16).float(), dim=-1, descending=True, stable=True).indices[:, :k]
+    topw = probs.gather(1, chosen)
+    topw = topw / topw.sum(-1, keepdim=True)
+    share = torch.bincount(chosen.reshape(-1), minlength=E).double() / chosen.numel()
+    aux = E * (share * probs.mean(0)).sum()
+    y = torch.zeros_like(x)
+    dx = torch.zeros_like(x)
+    dtopw = torch.zeros_like(topw)
+    dgu, dd = [], []
+    for e in range(E):
+        tok, slot = (chosen == e).nonzero(as_tuple=True)
+        xe = x.detach()[tok].requires_grad_()
+        gu = layer.w_gate_up[e].detach().double().requires_grad_()
+        down = layer.w_down[e].detach().double().requires_grad_()
+        we = topw.detach()[tok, slot].requires_grad_()
+        g, u = (xe @ gu.T).split(f, dim=1)
+        ye = (torch.nn.functional.silu(g) * u) @ down.T * we[:, None]
+        gx, gw, ggu, gd = torch.autograd.grad(ye, [xe, we, gu, down], dy[tok])
+        y = y.index_add(0, tok, ye.detach())
+        dx = dx.index_add(0, tok, gx)
+        dtopw[tok, slot] = gw
+        dgu.append(ggu.float())  # 2.8 GB an expert in 64 bits
+        dd.append(gd.float())
+    rx, drouter = torch.autograd.grad([topw, aux], [x, router], [dtopw, torch.full_like(aux, layer.aux_coef)])
+    grads = [drouter.float().reshape(-1)] + [g.reshape(-1) for g in dgu] + [g.reshape(-1) for g in dd]
+    return dict(y=y, aux=aux.detach(), dx=dx + rx, dweights=torch.cat(grads))
+
+
+def exact(case, seed):
+    c, kind, state = case, case["kind"], prepare(case, seed)
+    if kind in ("llama", "gpt2"):
+        return _step64(c, state)
+    if kind == "score":
+        with torch.no_grad():
+            w = {n: p.double() for n, p in state["model"].named_parameters()}
+            logits = _llama64(c, w, state["ids"])
+            loss = torch.nn.functional.cross_entropy(logits, state["target"].reshape(-1))
+            return dict(logits=logits.view(c["batch"], c["seq"], -1), loss=loss)
+    if kind == "attention":
+        qkv = state["qkv"].detach().double().requires_grad_()
+        out = _attention64(qkv, c["seq"], c["heads"], c["kv_heads"], c["head_dim"], c["rotary"])
+        (dqkv,) = torch.autograd.grad(out, qkv, state["dout"].double())
+        return dict(out=out.detach(), dqkv=dqkv)
+    if kind == "head":
+        h = state["h"].detach().double().requires_grad_()
+        weight = state["weight"].detach().double().requires_grad_()
+        loss = torch.nn.functional.cross_entropy((h @ weight.T)[:, : c["vocab"]], state["target"])
+        dh, dw = torch.autograd.grad(loss, [h, weight])
+        return dict(loss=loss.detach(), dh=dh, dweight=dw.reshape(-1))
+    if kind == "moe":
+        return _moe64(c, state)
+    opt = state["opt"]
+    flat = opt.groups[0]
+    master = opt.master[0]
+    w = flat.data.double() if master is None else master.double()
+    w, m, v = _adamw64(w, flat.grad.double() * 0.5, opt.lr, opt.betas, opt.eps, opt.weight_decay)
+    return dict(weights=w, m=m, v=v, master=None if master is None else w)
