@@ -294,8 +294,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       __syncthreads_and(ok);
     }
   } else if (warp == 0) {
-    // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    // ------------------------------------------------------------ TMA producer (whole warp, one elected lane issues)
+    {
       uint32_t stage = 0, phase = 0;
       bool ok = true;
       const uint32_t full0_remote = (kCtaGroup == 2) ? mapa_u32(smem_u32(&full[0]), 0) : 0;
@@ -323,56 +323,62 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           }
         }
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag)) {
-            ok = false;
-            break;
-          }
+          ok = __all_sync(0xffffffffu, mbar_wait(&empty[stage], phase ^ 1, abort_flag));
+          if (!ok) break;
           uint8_t* a_dst = sA + stage * A_BYTES;
           uint8_t* b_dst = sB + stage * B_BYTES;
           const int k0 = kb * BK;
-          if constexpr (kCtaGroup == 1) {
-            mbar_expect_tx(&full[stage], STAGE_BYTES);
-            if (!p.a_mn) {
-              tma_load_2d(a_dst, tma_a, &full[stage], k0, m0);
-            } else {
+          if (elect_one()) {
+            if constexpr (kCtaGroup == 1) {
+              mbar_expect_tx(&full[stage], STAGE_BYTES);
+              if (!p.a_mn) {
+                tma_load_2d(a_dst, tma_a, &full[stage], k0, m0);
+              } else {
 #pragma unroll
-              for (int i = 0; i < BM_CTA / 64; ++i) tma_load_2d(a_dst + i * 8192, tma_a, &full[stage], m0 + i * 64, k0);
-            }
-            if (!p.b_mn) {
-              tma_load_2d(b_dst, &tmB, &full[stage], k0, n0 + bn_off);
-            } else {
+                for (int i = 0; i < BM_CTA / 64; ++i) tma_load_2d(a_dst + i * 8192, tma_a, &full[stage], m0 + i * 64, k0);
+              }
+              if (!p.b_mn) {
+                tma_load_2d(b_dst, &tmB, &full[stage], k0, n0 + bn_off);
+              } else {
 #pragma unroll
-              for (int i = 0; i < BN_CTA / 64; ++i)
-                tma_load_2d(b_dst + i * 8192, &tmB, &full[stage], n0 + i * 64, k0 + bk_off);
-            }
-          } else {
-            if (leader) mbar_expect_tx(&full[stage], STAGE_BYTES * 2);
-            const uint32_t bar = full0_remote + stage * 8;
-            if (!p.a_mn) {
-              tma_load_2d_pair(a_dst, tma_a, bar, k0, m0);
+                for (int i = 0; i < BN_CTA / 64; ++i)
+                  tma_load_2d(b_dst + i * 8192, &tmB, &full[stage], n0 + i * 64, k0 + bk_off);
+              }
             } else {
+              if (leader) mbar_expect_tx(&full[stage], STAGE_BYTES * 2);
+              const uint32_t bar = full0_remote + stage * 8;
+              if (!p.a_mn) {
+                tma_load_2d_pair(a_dst, tma_a, bar, k0, m0);
+              } else {
 #pragma unroll
-              for (int i = 0; i < BM_CTA / 64; ++i) tma_load_2d_pair(a_dst + i * 8192, tma_a, bar, m0 + i * 64, k0);
-            }
-            if (!p.b_mn) {
-              tma_load_2d_pair(b_dst, &tmB, bar, k0, n0 + bn_off);
-            } else {
+                for (int i = 0; i < BM_CTA / 64; ++i) tma_load_2d_pair(a_dst + i * 8192, tma_a, bar, m0 + i * 64, k0);
+              }
+              if (!p.b_mn) {
+                tma_load_2d_pair(b_dst, &tmB, bar, k0, n0 + bn_off);
+              } else {
 #pragma unroll
-              for (int i = 0; i < BN_CTA / 64; ++i)
-                tma_load_2d_pair(b_dst + i * 8192, &tmB, bar, n0 + i * 64, k0 + bk_off);
+                for (int i = 0; i < BN_CTA / 64; ++i)
+                  tma_load_2d_pair(b_dst + i * 8192, &tmB, bar, n0 + i * 64, k0 + bk_off);
+              }
             }
           }
+          __syncwarp();
           if (++stage == kStages) {
             stage = 0;
             phase ^= 1;
           }
         }
       }
-      if (!ok) atomicExch(p.err, ERR_WAIT_TIMEOUT);
+      if (!ok && lane == 0) atomicExch(p.err, ERR_WAIT_TIMEOUT);
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0 && leader) {
+    // The whole warp walks the loop (waits included) so that control flow stays warp-uniform; one elected lane issues.
+    // Under `lane == 0` issuing set the pace: a 64-deep k-block took 512 to 570 cycles with every tile shape, although
+    // its four MMAs run in 256 (128 x 128 tiles).  Elected in both issuing warps, of this kernel on a B200:
+    // 4096 x 4096 x 8192 weight gradient 235 -> 224 us, 8192 x 4096 x 4096 207 -> 201 us, 77 x 4096 x 4096 26.4 -> 23.7 us;
+    // a k-block takes 407 to 505 cycles, about what its operands take to arrive.
+    if (leader) {
       const uint32_t idesc = make_idesc_bf16(BM_CTA * kCtaGroup, BN, p.a_mn, p.b_mn);
       // K-major: 16 k-elements = 32 B inside the swizzled row; MN-major: 16 k-rows of 128 B
       const uint32_t a_kstep = p.a_mn ? 2048 : 32;
@@ -385,40 +391,41 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         int tn_, row0_, ml_, grp_, kb0, kb1;
         locate(tile, tn_, row0_, ml_, grp_, kb0, kb1);
         if (kb1 <= kb0) continue;  // empty group: no accumulator is produced, the epilogue skips the tile too
-        if (!mbar_wait(&tempty[acc], acc_phase ^ 1, abort_flag)) {
-          ok = false;
-          break;
-        }
+        ok = __all_sync(0xffffffffu, mbar_wait(&tempty[acc], acc_phase ^ 1, abort_flag));
+        if (!ok) break;
         tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + acc * BN;
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(&full[stage], phase, abort_flag)) {
-            ok = false;
-            break;
-          }
+          ok = __all_sync(0xffffffffu, mbar_wait(&full[stage], phase, abort_flag));
+          if (!ok) break;
           tc_fence_after_sync();
-          const uint32_t a_addr = smem_u32(sA + stage * A_BYTES);
-          const uint32_t b_addr = smem_u32(sB + stage * B_BYTES);
+          const uint64_t da = make_smem_desc(smem_u32(sA + stage * A_BYTES), a_lbo, 1024);
+          const uint64_t db = make_smem_desc(smem_u32(sB + stage * B_BYTES), b_lbo, 1024);
+          if (elect_one()) {
+            // descriptors of the steps differ only in the start address (low 14 bits, in 16-byte units)
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            const uint64_t da = make_smem_desc(a_addr + k * a_kstep, a_lbo, 1024);
-            const uint64_t db = make_smem_desc(b_addr + k * b_kstep, b_lbo, 1024);
-            umma_ss<kCtaGroup>(d_tmem, da, db, idesc, (kb != kb0) || (k != 0));
+            for (int k = 0; k < BK / 16; ++k)
+              umma_ss<kCtaGroup>(d_tmem, da + ((k * a_kstep) >> 4), db + ((k * b_kstep) >> 4), idesc,
+                                 (kb != kb0) || (k != 0));
+            if constexpr (kCtaGroup == 1) umma_commit(&empty[stage]);
+            else umma_commit_pair(&empty[stage], 3);
           }
-          if constexpr (kCtaGroup == 1) umma_commit(&empty[stage]);
-          else umma_commit_pair(&empty[stage], 3);
+          __syncwarp();
           if (++stage == kStages) {
             stage = 0;
             phase ^= 1;
           }
         }
         if (!ok) break;
-        if constexpr (kCtaGroup == 1) umma_commit(&tfull[acc]);
-        else umma_commit_pair(&tfull[acc], 3);
+        if (elect_one()) {
+          if constexpr (kCtaGroup == 1) umma_commit(&tfull[acc]);
+          else umma_commit_pair(&tfull[acc], 3);
+        }
+        __syncwarp();
         acc ^= 1;
         if (acc == 0) acc_phase ^= 1;
       }
-      if (!ok) atomicExch(p.err, ERR_WAIT_TIMEOUT);
+      if (!ok && lane == 0) atomicExch(p.err, ERR_WAIT_TIMEOUT);
     }
   } else {
     // ------------------------------------------------------------ epilogue
