@@ -56,6 +56,29 @@ def test_gemm_epilogues(variant):
     assert _rel(acc, r0 + 1) < 1e-4
 
 
+@pytest.mark.parametrize("variant", [1, 2, 3])
+@pytest.mark.parametrize("M,N", [(77, 1000), (300, 256), (257, 288), (33, 40)])
+def test_gemm_epilogue_edges(variant, M, N):
+    """Rows that end inside a warp's 32, columns that end inside a 32-column chunk, one chunk and odd chunk counts: the
+    operands the epilogue fetches ahead (residual, fp32 target) have to belong to the rows and columns it writes."""
+    from pippy_b200.ops.gemm import gemm
+
+    K = 192
+    a, b, bias, res = _bf16(M, K), _bf16(N, K), _bf16(N), _bf16(M, N)
+    r0 = a.float() @ b.float().t()
+    assert _rel(gemm(a, b, bias=bias, residual=res, variant=variant), r0 + bias.float() + res.float()) < 1e-2
+    acc0 = torch.randn(M + 1, N, device="cuda")  # one guard row
+    acc = acc0.clone()
+    gemm(a, b, out=acc[:M], accumulate=True, variant=variant)
+    assert _rel(acc[:M], acc0[:M] + r0) < 1e-4 and torch.equal(acc[M], acc0[M])
+    gemm(a, b, bias=bias, residual=res, out=acc[:M], accumulate=True, variant=variant)
+    assert _rel(acc[:M], acc0[:M] + 2 * r0 + bias.float() + res.float()) < 1e-4
+    aux = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+    out = gemm(a, b, bias=bias, residual=res, act=1, aux=aux, variant=variant)
+    assert _rel(out, F.gelu(r0 + bias.float(), approximate="tanh") + res.float()) < 1e-2
+    assert _rel(aux, r0 + bias.float()) < 1e-2
+
+
 @pytest.mark.parametrize("H", [768, 4096, 5120])
 @pytest.mark.parametrize("layer", [False, True])
 def test_norm(H, layer):
