@@ -472,31 +472,25 @@ class _CrossEntropyFn(torch.autograd.Function):
     def forward(ctx, logits, targets, vocab: int, reduction: str, ignore_index: int, inplace: bool):
         T, ld = logits.shape
         tgt = targets.reshape(-1).contiguous()
-        loss_rows = torch.empty(T, dtype=torch.float32, device=logits.device)
-        dlogits = logits if inplace else torch.empty_like(logits)
-        if reduction == "mean":
-            n_valid = (tgt != ignore_index).sum().clamp(min=1).to(torch.float32)
-        else:
-            n_valid = None
+        dev = logits.device
+        loss_rows = torch.empty(T, dtype=torch.float32, device=dev)
+        # the gradient is formed with the loss, where anyone wants it (`inplace` promises it in `logits`)
+        dlogits = logits if inplace else (torch.empty_like(logits) if ctx.needs_input_grad[0] else None)
+        n_valid = torch.empty((), dtype=torch.float32, device=dev) if reduction == "mean" else None
+        loss = torch.empty((), dtype=torch.float32, device=dev)
         _lib.check(
-            _lib.lib().pb_xent_fwd_bwd(_lib.ptr(logits), _lib.ptr(dlogits), _lib.ptr(tgt), _lib.ptr(loss_rows),
-                                       _lib.c_ll(T), _lib.c_int(vocab), _lib.c_ll(logits.stride(0)),
-                                       _lib.c_float(1.0), _lib.c_ll(ignore_index), _lib.stream_ptr()),
-            "pb_xent_fwd_bwd",
+            _lib.lib().pb_xent(_lib.ptr(logits), _lib.ptr(dlogits), _lib.ptr(tgt), _lib.ptr(loss_rows),
+                               _lib.ptr(n_valid), _lib.ptr(loss), _lib.c_ll(T), _lib.c_int(vocab),
+                               _lib.c_ll(logits.stride(0)), _lib.c_ll(ignore_index), _lib.stream_ptr()),
+            "pb_xent",
         )
-        loss = loss_rows.sum()
-        if n_valid is not None:
-            loss = loss / n_valid
-        ctx.save_for_backward(dlogits, n_valid)
+        ctx.save_for_backward(dlogits)
         return loss
 
     @staticmethod
     def backward(ctx, dloss):
-        dlogits, n_valid = ctx.saved_tensors
-        scale = dloss.to(torch.float32).reshape(1)
-        if n_valid is not None:
-            scale = scale / n_valid
-        scale = scale.contiguous()
+        (dlogits,) = ctx.saved_tensors
+        scale = dloss.to(torch.float32).reshape(1).contiguous()
         _lib.check(
             _lib.lib().pb_scale_bf16(_lib.ptr(dlogits), _lib.ptr(scale), _lib.c_ll(dlogits.numel()),
                                      _lib.stream_ptr()),

@@ -223,6 +223,39 @@ def test_cross_entropy():
     assert logits.grad[:, V:].abs().max().item() == 0
 
 
+@pytest.mark.parametrize("V,pad", [(8, 0), (13, 3), (4096, 0), (4097, 7), (32000, 0), (50257, 47), (56000, 8), (56001, 7)])
+@pytest.mark.parametrize("reduction", ["mean", "sum"])
+def test_cross_entropy_class_counts(V, pad, reduction):
+    """Around the class counts at which another kernel takes the row (4096, 56000) and around whole 16-byte vectors:
+    loss, gradient (with an incoming gradient of 1 and of 3), ignored rows, columns at and beyond the padding, and the
+    loss alone without a gradient."""
+    from pippy_b200.ops import functional as pf
+
+    T = 37
+    logits = _bf16(T, V + pad, scale=3.0)
+    logits[:, V:] = 1e4  # padding has to have no influence
+    tgt = torch.randint(0, V, (T,), device="cuda")
+    tgt[3], tgt[4], tgt[0] = -100, V - 1, 0
+    lf = logits[:, :V].double().requires_grad_()
+    ref = F.cross_entropy(lf, tgt, reduction=reduction, ignore_index=-100)
+    ref.backward()
+    for factor in (1.0, 3.0):
+        x = logits.clone().requires_grad_()
+        loss = pf.cross_entropy(x, tgt, vocab_size=V, reduction=reduction)
+        assert abs(loss.item() - ref.item()) < 1e-5 * abs(ref.item())
+        (loss * factor).backward()
+        # one rounding to bf16 (relative 2^-8 at most), a second one with a factor, and 1e-4 for fp32 exponentials
+        bound = (2 ** -8 if factor == 1.0 else 2 ** -7) + 1e-4
+        assert ((x.grad[:, :V].double() - factor * lf.grad).abs() <= bound * factor * lf.grad.abs() + 1e-9).all()
+        assert x.grad[3].abs().max().item() == 0 and (pad == 0 or x.grad[:, V:].abs().max().item() == 0)
+    keep = logits.clone()
+    with torch.no_grad():
+        assert torch.equal(pf.cross_entropy(logits, tgt, vocab_size=V, reduction=reduction), loss.detach())
+        assert torch.equal(logits, keep)
+        pf.cross_entropy(logits, tgt, vocab_size=V, reduction=reduction, inplace=True)
+        assert ((logits[:, :V].double() - lf.grad).abs() <= (2 ** -8 + 1e-4) * lf.grad.abs() + 1e-9).all()
+
+
 def test_embedding():
     from pippy_b200.ops import functional as pf
 
