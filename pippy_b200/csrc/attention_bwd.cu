@@ -52,6 +52,7 @@ struct BwdParams {
   int B, S, Hq, Hkv;
   float scale, scale_log2;
   int causal;
+  int head_group;
   int* err;
 };
 
@@ -96,7 +97,10 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant__ 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int G = p.Hq / p.Hkv;
-  const int b = blockIdx.z;
+  const int heads = kMode == 0 ? p.Hkv : p.Hq;
+  const int res_tiles = (p.S + BR - 1) / BR;
+  const TileOrder order = tile_order(blockIdx.x, res_tiles, heads * p.B, p.head_group);
+  const int b = order.index / heads;
   const int row_base = b * p.S;
 
   // ---- work decomposition
@@ -105,18 +109,15 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant__ 
   int hkv;
   int blk_start, nblk_per_head, n_it;
   if (kMode == 0) {
-    const int kt = blockIdx.x;
-    r0 = kt * BR;
-    hkv = blockIdx.y;
+    r0 = order.tile_rank * BR;  // the first keys are seen by the most queries
+    hkv = order.index - b * heads;
     head_res = hkv;
     blk_start = p.causal ? (r0 / BS) : 0;
     nblk_per_head = (p.S + BS - 1) / BS - blk_start;
     n_it = G * nblk_per_head;
   } else {
-    const int nqt = (p.S + BR - 1) / BR;
-    const int qt = nqt - 1 - blockIdx.x;
-    r0 = qt * BR;
-    head_res = blockIdx.y;
+    r0 = (res_tiles - 1 - order.tile_rank) * BR;
+    head_res = order.index - b * heads;
     hkv = head_res / G;
     blk_start = 0;
     const int kv_end = p.causal ? min(p.S, r0 + BR) : p.S;
@@ -517,7 +518,7 @@ __global__ void __launch_bounds__(256) fa_delta_kernel(const __nv_bfloat16* __re
 
 template <int D, int kMode>
 static int launch_bwd(const CUtensorMap& x1, const CUtensorMap& x2, const CUtensorMap& y1, const CUtensorMap& y2,
-                      const BwdParams& p, cudaStream_t stream) {
+                      BwdParams p, cudaStream_t stream) {
   constexpr int NCH = D / 64;
   constexpr int SMEM = 2 * NCH * 128 * 128 + 2 * NST * NCH * 64 * 128 + 2048 + 256;
   auto kern = fa_bwd_kernel<D, kMode>;
@@ -527,7 +528,9 @@ static int launch_bwd(const CUtensorMap& x1, const CUtensorMap& x2, const CUtens
     if (e != cudaSuccess) return (int)e;
     attr_set = true;
   }
-  dim3 grid((p.S + BR - 1) / BR, kMode == 0 ? p.Hkv : p.Hq, p.B);
+  const int tiles = (p.S + BR - 1) / BR, heads = (kMode == 0 ? p.Hkv : p.Hq) * p.B;
+  p.head_group = attention_head_group(tiles, heads);
+  const unsigned grid = (unsigned)tiles * heads;
   kern<<<grid, kThreads, SMEM, stream>>>(x1, x2, y1, y2, p);
   pb_count_launch(1);
   return (int)cudaGetLastError();
