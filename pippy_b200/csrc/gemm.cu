@@ -74,6 +74,13 @@ struct GemmParams {
   const int* group_start;
   int b_group_stride;
   long long c_group_stride;
+  // ---- split contraction (plain GEMMs): tiles from `dp_tiles` on are cut into `splits` ranges of k-blocks, one work
+  // item each.  Every item leaves its fp32 partial tile in `split_ws`; the one that arrives last at the tile's counter
+  // (per 32 rows) adds the partials in range order, so the result does not depend on which one that was, and runs
+  // the epilogue.  Nobody waits.  The counters are zero before and after every launch.
+  int dp_tiles, splits;
+  float* split_ws;
+  int* split_counters;
 };
 
 constexpr int MAX_GROUPS = 8;
@@ -212,7 +219,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   // grouped mode 1 only knows its M tiles now; mode 2 runs the full [M, N] tile grid once per group
   const int num_m_tiles = (p.grouped == 1) ? gt->prefix[MAX_GROUPS] : p.num_m_tiles;
   const int tiles_per_group = num_m_tiles * p.num_n_tiles;
-  const int num_tiles = (p.grouped == 2) ? tiles_per_group * p.n_groups : tiles_per_group;
+  // work items: whole tiles, then the ranges of the split ones
+  const int num_tiles = (p.grouped == 2)   ? tiles_per_group * p.n_groups
+                        : (p.splits > 1) ? p.dp_tiles + (tiles_per_group - p.dp_tiles) * p.splits
+                                         : tiles_per_group;
   constexpr int TILE_M_ALL = BM_CTA * kCtaGroup;
   // Where a tile lives.  Every role calls this with the same arguments, so all agree on the rows, the group and
   // the contraction range (kb0 <= kb < kb1; an empty range means the tile is skipped by everybody).
@@ -221,6 +231,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     grp = 0;
     kb0 = 0;
     kb1 = p.num_k_blocks;
+    if (p.splits > 1 && tile >= p.dp_tiles) {
+      const int item = tile - p.dp_tiles, range = item % p.splits;
+      tile = p.dp_tiles + item / p.splits;
+      kb0 = (int)((long long)p.num_k_blocks * range / p.splits);
+      kb1 = (int)((long long)p.num_k_blocks * (range + 1) / p.splits);
+    }
     if (p.grouped == 2) {
       grp = tile / tiles_per_group;
       tile -= grp * tiles_per_group;
@@ -509,7 +525,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       // residual 19.7 -> 12.6 us, 8192 x 4096 x 4096 201 -> 182 us (1 510 TFLOP/s).
       const int row_w = row - lane;  // first of this warp's 32 rows
       const bool fast = vec_ok && p.fused != 2 && row_w + 32 <= m_limit;
-      const int fast_chunks = fast ? min(BN, p.N - n0) / 32 : 0;
+      int fast_chunks = fast ? min(BN, p.N - n0) / 32 : 0;
       const bool acc_c = p.accumulate && p.out_fp32 && p.residual == nullptr && p.bias == nullptr && p.act == 0;
       const bool plain_bf16 = !p.out_fp32 && p.residual == nullptr && p.act == 0;
       const bool res_bf16 = !p.out_fp32 && p.residual != nullptr && p.act == 0;
@@ -529,11 +545,80 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       tc_fence_after_sync();
       const uint32_t t_row = tmem_base + acc * BN + (static_cast<uint32_t>(quarter * 32) << 16);
       int c_done = 0;
+      // split tile: partials of one warp's 32 rows lie as [chunk][float4 of the row][lane], so that both the stores and
+      // the reads of a warp are contiguous
+      const bool is_split = p.splits > 1 && tile >= p.dp_tiles;
+      const int range = is_split ? (tile - p.dp_tiles) % p.splits : 0;
+      constexpr long long PART = 32 * BN;                       // floats of one warp's partial
+      constexpr long long ITEM = 4 * kCtaGroup * PART;          // floats of one work item
+      const float4* parts = nullptr;                            // this warp's partial of range 0
+      bool finish = true;
+      if (is_split) {
+        const int first_item = tile - p.dp_tiles - range;
+        const long long slot = (cta_rank * 4 + quarter) * PART;
+        parts = reinterpret_cast<const float4*>(p.split_ws + first_item * ITEM + slot);
+        finish = false;
+        if (row_w < m_limit) {
+          float4* own = reinterpret_cast<float4*>(p.split_ws + (first_item + range) * ITEM + slot);
+#pragma unroll 1
+          for (int c = 0; c < BN / 32 && n0 + c * 32 < p.N; ++c) {
+            uint32_t r[32];
+            tmem_ld_32x32(t_row + c * 32, r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+              __stcg(own + (c * 8 + q) * 32 + lane,
+                     make_float4(__uint_as_float(r[q * 4]), __uint_as_float(r[q * 4 + 1]),
+                                 __uint_as_float(r[q * 4 + 2]), __uint_as_float(r[q * 4 + 3])));
+          }
+          __threadfence();
+          __syncwarp();
+          int arrived = 0;
+          int* counter = p.split_counters + (first_item / p.splits) * (4 * kCtaGroup) + cta_rank * 4 + quarter;
+          if (lane == 0) arrived = atomicAdd(counter, 1);
+          arrived = __shfl_sync(0xffffffffu, arrived, 0);
+          finish = arrived == p.splits - 1;
+          if (finish) {
+            __threadfence();
+            if (lane == 0) *counter = 0;  // as the next launch expects it
+          }
+        }
+      }
+      if (!finish) {
+        c_done = BN / 32;
+        fast_chunks = 0;
+      }
+      // sum of the partials of chunk c in range order (this item's own ones are read back with the others)
+      auto gather = [&](int c, uint32_t(&r)[32]) {
+        float4 sum[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) sum[q] = __ldcg(parts + (c * 8 + q) * 32 + lane);
+        const float4* next = parts + ITEM / 4;
+#pragma unroll 3
+        for (int i = 1; i < p.splits; ++i, next += ITEM / 4) {
+          float4 t[8];
+#pragma unroll
+          for (int q = 0; q < 8; ++q) t[q] = __ldcg(next + (c * 8 + q) * 32 + lane);
+#pragma unroll
+          for (int q = 0; q < 8; ++q) sum[q] = add4(sum[q], t[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          r[q * 4] = __float_as_uint(sum[q].x);
+          r[q * 4 + 1] = __float_as_uint(sum[q].y);
+          r[q * 4 + 2] = __float_as_uint(sum[q].z);
+          r[q * 4 + 3] = __float_as_uint(sum[q].w);
+        }
+      };
       // this warp's 32 x 32 block of chunk c, turned: v[q] = columns [4 part, +4) of row 4 q + sub_row
       auto turned = [&](int c, float4(&v)[8]) {
         uint32_t r[32];
-        tmem_ld_32x32(t_row + c * 32, r);
-        tmem_ld_wait();
+        if (is_split) {
+          gather(c, r);
+        } else {
+          tmem_ld_32x32(t_row + c * 32, r);
+          tmem_ld_wait();
+        }
         float4* mine = reinterpret_cast<float4*>(stage_w + lane * 144);
 #pragma unroll
         for (int q = 0; q < 8; ++q)
@@ -642,8 +727,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const int col0 = n0 + c * 32;
         if (col0 >= p.N) break;  // uniform across the warp
         uint32_t r[32];
-        tmem_ld_32x32(t_row + c * 32, r);
-        tmem_ld_wait();
+        if (is_split) {
+          gather(c, r);
+        } else {
+          tmem_ld_32x32(t_row + c * 32, r);
+          tmem_ld_wait();
+        }
         if (zero_tail) {
           __nv_bfloat16* zp = reinterpret_cast<__nv_bfloat16*>(c_base) + (long long)row * p.ldc + col0;
           if (col0 + 32 <= p.N && vec_ok) {
@@ -897,7 +986,8 @@ static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParam
   p.group_m = kCtaGroup == 1 ? 16 : 8;
   if (g_group_m > 0 && !p.fused) p.group_m = g_group_m;
   // grouped M: up to one partial tile per group on top of the dense count (p.M is the buffers' row capacity)
-  const int tiles = (p.num_m_tiles + (p.grouped == 1 ? p.n_groups : 0)) * p.num_n_tiles * tile_multiplier;
+  int tiles = (p.num_m_tiles + (p.grouped == 1 ? p.n_groups : 0)) * p.num_n_tiles * tile_multiplier;
+  if (p.splits > 1) tiles = p.dp_tiles + (tiles - p.dp_tiles) * p.splits;
   int units = (sm_count - copy_ctas) / kCtaGroup;
   if (units > tiles) units = tiles;
   if (units < 1) units = 1;
@@ -929,6 +1019,64 @@ static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParam
 
 static int g_sm_reserve = 0;
 
+namespace {
+
+// How a plain GEMM is cut: kernel variant, tiles that run whole, ranges that each remaining tile is split into.
+struct GemmPlan {
+  int variant, dp_tiles, splits;
+  int items;  // split work items (0: no workspace needed)
+  double cycles;
+};
+
+constexpr long long SPLIT_ITEM_BYTES = 128 * 256 * 4;  // partial of one CTA, largest variant
+constexpr int SPLIT_COUNTERS = 1024;                   // 4 per CTA of a split tile, at most 148 CTAs
+
+// Estimated SM cycles of `variant` and the best split of its last wave.  Tiles run in waves of one per worker (CTA or
+// CTA pair).  When r tiles are left for the last wave they are cut into s ranges of k-blocks, r * s <= workers: the
+// wave takes 1/s of the time, plus the partial tiles' way through L2.
+//
+// Constants measured on a B200.  A 64-deep k-block takes about 480 cycles with 128 x 128 tiles, 640 with 128 x 256, 500
+// with pairs (what the operands take to arrive).  Start, first operands, last MMAs and the last tile's epilogue add
+// 7 000, 9 500 and 14 000.  Splitting costs 6 000 + 2 000 s with 128 x 128 tiles and 9 000 + 5 000 s with 256 columns.
+// Against the best unsplit variant, us: 77 x 4096 x 11008 46.1 -> 25.2 (s = 4), 77 x 4096 x 4096 20.6 -> 16.3 (4),
+// 2048 x 768 x 50304 192 -> 118 (3), 2999 x 5120 x 13824 321 -> 291 (4), 4096 x 4096 x 8192 205 -> 192 (2); on the other
+// side of the line 768 x 768 x 2048 14.4 -> 16.3 (3), 4095 x 4096 x 4096 97.1 -> 98.5 (2).  Variants where none is
+// split: 2048 x 768 x 768 11.4 with pairs, 8.6 with 128 x 128; 2048 x 50304 x 768 135 and 167.
+GemmPlan plan_variant(int variant, int M, int N, int K, int sms, bool may_split) {
+  const int ctas = variant == 2 ? 2 : 1, bn = variant == 3 ? 128 : 256;
+  const int units = sms / ctas;
+  const int tiles = ((M + 128 * ctas - 1) / (128 * ctas)) * ((N + bn - 1) / bn);
+  const int kb = (K + 63) / 64;
+  const double per_kb = variant == 2 ? 500 : (variant == 1 ? 640 : 480);
+  const double edge = variant == 2 ? 14000 : (variant == 1 ? 9500 : 7000);
+  const double split_fixed = variant == 3 ? 6000 : 9000, split_each = variant == 3 ? 2000 : 5000;
+  const int whole = tiles / units, rest = tiles - whole * units;
+  GemmPlan best{variant, tiles, 1, 0, edge + (whole + (rest ? 1 : 0)) * kb * per_kb};
+  if (may_split && rest) {
+    for (int s = 2; s <= 8 && rest * s <= units && s * 4 <= kb; ++s) {
+      const double c = edge + whole * kb * per_kb + ((kb + s - 1) / s) * per_kb + split_fixed + split_each * s;
+      if (c < 0.99 * best.cycles) best = GemmPlan{variant, whole * units, s, rest * s, c};
+    }
+  }
+  return best;
+}
+
+// The cheapest variant.  N <= 128 leaves half of a 256-column tile empty, M <= 128 the second CTA of a pair.
+GemmPlan plan_gemm(int M, int N, int K, int sms, bool may_split) {
+  GemmPlan plan = plan_variant(3, M, N, K, sms, may_split);
+  if (N > 128) {
+    const GemmPlan wide = plan_variant(1, M, N, K, sms, may_split);
+    if (wide.cycles < plan.cycles) plan = wide;
+    if (M > 128) {
+      const GemmPlan pair = plan_variant(2, M, N, K, sms, may_split);
+      if (pair.cycles < plan.cycles) plan = pair;
+    }
+  }
+  return plan;
+}
+
+}  // namespace
+
 extern "C" {
 
 // Leaves `n` SMs out of the persistent GEMM grid (for communication kernels that must run beside it).
@@ -942,9 +1090,26 @@ void pb_set_gemm_group_m(int n) { pb::g_group_m = n < 0 ? 0 : n; }
 // variant: 0 = automatic, 1 = single-CTA tiles (128 x 256), 2 = CTA-pair tiles (256 x 256),
 //          3 = single-CTA 128 x 128.
 // Returns 0 on success, a negative value for an argument error, a positive CUDA error otherwise.
-int pb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
-                 long long ldc, int a_mn, int b_mn, const void* bias, const void* residual, long long ldr, void* aux,
-                 int act, int out_fp32, int accumulate, int variant, int* err_dev, void* stream_) {
+// `split_ws`: pb_gemm_split_ws_bytes() bytes that no other stream uses, its last 4 KB (the counters) zero before the
+// first call and left zero by every call; null = the contraction is never split.  With `ask_ws` != 0 the call returns
+// PB_GEMM_WANTS_WS, without launching anything, where a split needs a workspace and none is given, or the given one
+// (which outlives the call) would become part of a graph under capture.
+#define PB_GEMM_WANTS_WS (-100)
+long long pb_gemm_split_ws_bytes() { return 148LL * SPLIT_ITEM_BYTES + SPLIT_COUNTERS * 4; }
+
+// out: variant, whole tiles, ranges per split tile, split work items
+void pb_gemm_plan(int M, int N, int K, int sms, int may_split, int* out) {
+  const GemmPlan plan = plan_gemm(M, N, K, sms, may_split != 0);
+  out[0] = plan.variant;
+  out[1] = plan.dp_tiles;
+  out[2] = plan.splits;
+  out[3] = plan.items;
+}
+
+int pb_gemm_bf16_ws(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
+                    long long ldc, int a_mn, int b_mn, const void* bias, const void* residual, long long ldr, void* aux,
+                    int act, int out_fp32, int accumulate, int variant, void* split_ws, int ask_ws, int* err_dev,
+                    void* stream_) {
   using namespace pb;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   if (M <= 0 || N <= 0 || K <= 0) return -1;
@@ -957,7 +1122,20 @@ int pb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, lon
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
   }
-  if (variant == 0) variant = (N <= 128) ? 3 : ((M >= 1024 && N >= 256) ? 2 : 1);
+  int sms = sm_count - g_sm_reserve;
+  if (sms < 2) sms = 2;
+  if (sms > 148) sms = 148;  // what the workspace is sized for
+  GemmPlan plan{variant, 0, 1, 0, 0.0};
+  if (variant == 0) {
+    plan = plan_gemm(M, N, K, sms, split_ws != nullptr || ask_ws);
+    if (plan.splits > 1 && ask_ws) {
+      cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+      cudaError_t e = split_ws ? cudaStreamIsCapturing(stream, &capture) : cudaSuccess;
+      if (e != cudaSuccess) return (int)e;
+      if (split_ws == nullptr || capture != cudaStreamCaptureStatusNone) return PB_GEMM_WANTS_WS;
+    }
+    variant = plan.variant;
+  }
   const int bn = (variant == 3) ? 128 : 256;
   const int b_rows = (variant == 2) ? bn / 2 : bn;
 
@@ -987,8 +1165,10 @@ int pb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, lon
   p.a_mn = a_mn;
   p.b_mn = b_mn;
   p.err = err_dev;
-  int sms = sm_count - g_sm_reserve;
-  if (sms < 2) sms = 2;
+  p.dp_tiles = plan.dp_tiles;
+  p.splits = plan.splits;
+  p.split_ws = reinterpret_cast<float*>(split_ws);
+  p.split_counters = reinterpret_cast<int*>(reinterpret_cast<char*>(split_ws) + 148LL * SPLIT_ITEM_BYTES);
   switch (variant) {
     case 1: return launch_gemm<1, 256, 4>(tmA, tmB, p, sms, stream);
     case 2: return launch_gemm<2, 256, 6>(tmA, tmB, p, sms, stream);
@@ -997,6 +1177,12 @@ int pb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, lon
   }
 }
 
+int pb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
+                 long long ldc, int a_mn, int b_mn, const void* bias, const void* residual, long long ldr, void* aux,
+                 int act, int out_fp32, int accumulate, int variant, int* err_dev, void* stream_) {
+  return pb_gemm_bf16_ws(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, bias, residual, ldr, aux, act, out_fp32,
+                         accumulate, variant, nullptr, 0, err_dev, stream_);
+}
 
 // Grouped GEMMs of a mixture-of-experts layer: ONE launch covers all local experts, and the group sizes stay on the
 // device (group_rows / group_start: int[n_groups] in device memory, group_start[g] a multiple of 256).

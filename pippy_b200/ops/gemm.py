@@ -1,12 +1,34 @@
 """Low-level wrapper of the tcgen05 GEMM kernel (``csrc/gemm.cu``)."""
 from __future__ import annotations
 
+from collections import OrderedDict
+
 import torch
 
 from . import _lib
 
 ACT_NONE = 0
 ACT_GELU_TANH = 1
+
+
+# Workspaces of the split contraction (partial tiles + arrival counters), one per device and stream: calls on a stream
+# run one after the other, and every call leaves the counters at zero for the next.  At most _MAX_SPLIT_WS are kept;
+# the allocator frees a dropped one in the order of the stream that used it.  A capture gets a workspace of its own,
+# which lives in the graph's pool and is cleared by the graph: a replay may run beside eager calls on the stream it was
+# captured on.
+_SPLIT_WS: "OrderedDict[tuple, torch.Tensor]" = OrderedDict()
+_MAX_SPLIT_WS = 8
+_WANTS_WS = -100
+_COUNTER_BYTES = 4096
+_lib.ON_DEVICE_ERROR.append(_SPLIT_WS.clear)  # a call that gave up may have left its counters behind
+
+
+def _new_split_ws(device: torch.device) -> torch.Tensor:
+    fn = _lib.lib().pb_gemm_split_ws_bytes
+    fn.restype = _lib.c_ll
+    ws = torch.empty(int(fn()), dtype=torch.uint8, device=device)
+    ws[-_COUNTER_BYTES:].zero_()
+    return ws
 
 
 def gemm(
@@ -51,18 +73,32 @@ def gemm(
         assert residual.shape == (M, N) and residual.stride(1) == 1 and residual.dtype == torch.bfloat16
     if aux is not None:
         assert aux.shape == (M, N) and aux.stride(0) == out.stride(0) and aux.dtype == torch.bfloat16
-    rc = _lib.lib().pb_gemm_bf16(
-        _lib.ptr(a), _lib.ptr(b), _lib.ptr(out),
-        _lib.c_int(M), _lib.c_int(N), _lib.c_int(K),
-        _lib.c_ll(a.stride(0)), _lib.c_ll(b.stride(0)), _lib.c_ll(out.stride(0)),
-        _lib.c_int(int(a_mn)), _lib.c_int(int(b_mn)),
-        _lib.ptr(bias), _lib.ptr(residual), _lib.c_ll(residual.stride(0) if residual is not None else 0),
-        _lib.ptr(aux), _lib.c_int(act), _lib.c_int(int(out_fp32)), _lib.c_int(int(accumulate)),
-        _lib.c_int(variant), _lib.ptr(_lib.err_word(a.device)), _lib.stream_ptr(),
-    )
+    stream = _lib.stream_ptr()
+    key = (a.device.index, stream.value)
+    ws = _SPLIT_WS.get(key)
+
+    def call(ws, ask):
+        return _lib.lib().pb_gemm_bf16_ws(
+            _lib.ptr(a), _lib.ptr(b), _lib.ptr(out),
+            _lib.c_int(M), _lib.c_int(N), _lib.c_int(K),
+            _lib.c_ll(a.stride(0)), _lib.c_ll(b.stride(0)), _lib.c_ll(out.stride(0)),
+            _lib.c_int(int(a_mn)), _lib.c_int(int(b_mn)),
+            _lib.ptr(bias), _lib.ptr(residual), _lib.c_ll(residual.stride(0) if residual is not None else 0),
+            _lib.ptr(aux), _lib.c_int(act), _lib.c_int(int(out_fp32)), _lib.c_int(int(accumulate)),
+            _lib.c_int(variant), _lib.ptr(ws), _lib.c_int(ask), _lib.ptr(_lib.err_word(a.device)), stream,
+        )
+
+    rc = call(ws, 1)
+    if rc == _WANTS_WS:  # none kept for this stream, or the stream is being captured
+        ws = _new_split_ws(a.device)
+        if not torch.cuda.is_current_stream_capturing():
+            _SPLIT_WS[key] = ws
+            while len(_SPLIT_WS) > _MAX_SPLIT_WS:
+                _SPLIT_WS.popitem(last=False)
+        rc = call(ws, 0)
     if rc != 0:
         raise _lib.KernelError(
-            f"pb_gemm_bf16 failed with code {rc}: a {tuple(a.shape)} strides {a.stride()} ptr%16={a.data_ptr() % 16}, "
+            f"pb_gemm_bf16_ws failed with code {rc}: a {tuple(a.shape)} strides {a.stride()} ptr%16={a.data_ptr() % 16}, "
             f"b {tuple(b.shape)} strides {b.stride()} ptr%16={b.data_ptr() % 16}, out {tuple(out.shape)} "
             f"{out.dtype} strides {out.stride()}, a_mn={a_mn} b_mn={b_mn}, M={M} N={N} K={K}")
     return out

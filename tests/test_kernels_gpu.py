@@ -79,6 +79,42 @@ def test_gemm_epilogue_edges(variant, M, N):
     assert _rel(aux, r0 + bias.float()) < 1e-2
 
 
+@pytest.mark.parametrize("M,N,K", [(77, 4096, 4096), (1, 256, 8192), (700, 1000, 4096), (2048, 768, 16384), (2500, 2600, 8200)])
+def test_gemm_split_contraction(M, N, K):
+    """Shapes whose last wave is split over ranges of the contraction: every epilogue, the same bits each time, another
+    stream at the same time, and a captured call that is replayed beside eager ones."""
+    import ctypes
+
+    from pippy_b200.ops import _lib
+    from pippy_b200.ops.gemm import gemm
+
+    plan = (ctypes.c_int * 4)()
+    _lib.lib().pb_gemm_plan(M, N, K, 148, 1, plan)
+    assert plan[2] > 1, list(plan)
+    a, b, bias, res = _bf16(M, K), _bf16(K, N), _bf16(N), _bf16(M, N)
+    ref = a.float() @ b.float()
+    out = gemm(a, b, b_mn=True)
+    assert _rel(out, ref) < 1e-2
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        others = [gemm(a, b, b_mn=True) for _ in range(4)]
+    again = [gemm(a, b, b_mn=True) for _ in range(4)]
+    torch.cuda.current_stream().wait_stream(side)
+    assert all(torch.equal(out, o) for o in others + again)
+    assert _rel(gemm(a, b, b_mn=True, bias=bias, residual=res), ref + bias.float() + res.float()) < 1e-2
+    acc = torch.ones(M, N, device="cuda")
+    gemm(a, b, b_mn=True, out=acc, accumulate=True)
+    assert _rel(acc, ref + 1) < 1e-4
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = gemm(a, b, b_mn=True)
+    for _ in range(2):
+        graph.replay()
+        assert torch.equal(gemm(a, b, b_mn=True), out)
+        assert torch.equal(captured, out)
+
+
 @pytest.mark.parametrize("H", [768, 4096, 5120])
 @pytest.mark.parametrize("layer", [False, True])
 def test_norm(H, layer):
