@@ -28,6 +28,33 @@ c_ll = ctypes.c_longlong
 c_float = ctypes.c_float
 
 
+# Argument types of the functions that the ops call with plain Python numbers (:func:`addr`, :func:`stream_addr`):
+# p pointer, i int, l long long, f float.  With them declared ctypes converts the numbers itself, which costs a
+# fraction of building a ctypes object per argument (a GEMM call has 23).
+SIGNATURES = {
+    "pb_accum_bf16_into_f32": "pplp",
+    "pb_adamw": "ppppplfffffifip",
+    "pb_colsum_bf16": "pplilp",
+    "pb_embed_bwd": "pppplii" "lp",
+    "pb_embed_fwd": "pppplii" "lp",
+    "pb_flash_bwd": "p" * 10 + "iiiii" "llllll" "fipp",
+    "pb_flash_fwd": "ppppp" "iiiii" "llll" "fipp",
+    "pb_gelu_bwd": "ppplp",
+    "pb_gemm_bf16_ws": "ppp" "iii" "lll" "ii" "pplp" "iii" "i" "pi" "pp",
+    "pb_norm_bwd_res": "p" * 11 + "ip" "iiii" "p",
+    "pb_norm_bwd_scratch_floats": "ii",
+    "pb_norm_fwd": "p" * 6 + "iifip",
+    "pb_rope": "ppp" "liii" "lfp",
+    "pb_scale_bf16": "pplp",
+    "pb_set_gemm_group_m": "i",
+    "pb_set_sm_reserve": "i",
+    "pb_swiglu_bwd": "ppplipp",
+    "pb_swiglu_fwd": "pplipp",
+    "pb_xent": "p" * 6 + "lill" "p",
+}
+_TYPES = {"p": c_void_p, "i": c_int, "l": c_ll, "f": c_float}
+
+
 class KernelError(RuntimeError):
     """A kernel of this library reported a failure (bad argument, CUDA error, bounded wait ran out)."""
 
@@ -47,6 +74,8 @@ def lib() -> ctypes.CDLL:
         handle = ctypes.CDLL(LIB_PATH)
         handle.pb_launch_count.restype = c_ll
         handle.pb_last_cuda_error.restype = ctypes.c_char_p
+        for name, types in SIGNATURES.items():
+            getattr(handle, name).argtypes = [_TYPES[t] for t in types]
         _LIB = handle
     return _LIB
 
@@ -63,6 +92,17 @@ def stream_ptr() -> c_void_p:
     return c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
+def addr(t: torch.Tensor | None) -> int | None:
+    """Data pointer as a plain number, for the functions of :data:`SIGNATURES` only: without declared types ctypes
+    passes a Python int as a 32-bit one."""
+    return None if t is None else t.data_ptr()
+
+
+def stream_addr() -> int:
+    """The current stream of the current device as a plain number (:data:`SIGNATURES` functions only)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
 def err_word(device: torch.device | None = None) -> torch.Tensor:
     """Per-device int32 word that kernels set when a bounded wait runs out."""
     idx = torch.cuda.current_device() if device is None or device.index is None else device.index
@@ -74,6 +114,12 @@ def err_word(device: torch.device | None = None) -> torch.Tensor:
             # debug build: kernels without an error-word argument of their own report through this one
             lib().pb_set_debug_err_ptr(c_void_p(w.data_ptr()))
     return w
+
+
+def err_addr(device: torch.device) -> int:
+    """Data pointer of :func:`err_word` as a plain number (:data:`SIGNATURES` functions only)."""
+    w = _ERR_WORDS.get(device.index)
+    return (err_word(device) if w is None else w).data_ptr()
 
 
 def bounds_check_enabled() -> bool:

@@ -48,8 +48,8 @@ def _accumulate_param_grad(param: torch.Tensor, grad: torch.Tensor) -> None:
     if mg is not None:
         if grad.dtype == torch.bfloat16 and mg.dtype == torch.float32 and grad.is_cuda and grad.numel() % 8 == 0:
             _lib.check(
-                _lib.lib().pb_accum_bf16_into_f32(_lib.ptr(mg), _lib.ptr(grad.contiguous()), _lib.c_ll(grad.numel()),
-                                                  _lib.stream_ptr()),
+                _lib.lib().pb_accum_bf16_into_f32(_lib.addr(mg), _lib.addr(grad.contiguous()), grad.numel(),
+                                                  _lib.stream_addr()),
                 "pb_accum_bf16_into_f32",
             )
         else:
@@ -85,8 +85,8 @@ def _wgrad(dy2: torch.Tensor, x2: torch.Tensor, weight: torch.Tensor, bias: Opti
         else:
             target = torch.zeros(bias.shape, dtype=torch.float32, device=bias.device)
         _lib.check(
-            _lib.lib().pb_colsum_bf16(_lib.ptr(dy2), _lib.ptr(target), _lib.c_ll(dy2.shape[0]),
-                                      _lib.c_int(dy2.shape[1]), _lib.c_ll(dy2.stride(0)), _lib.stream_ptr()),
+            _lib.lib().pb_colsum_bf16(_lib.addr(dy2), _lib.addr(target), dy2.shape[0],
+                                      dy2.shape[1], dy2.stride(0), _lib.stream_addr()),
             "pb_colsum_bf16",
         )
         if target is not bmg:
@@ -136,8 +136,8 @@ class _LinearFn(torch.autograd.Function):
         if ctx.act == ACT_GELU_TANH:
             dpre = torch.empty_like(dy2)
             _lib.check(
-                _lib.lib().pb_gelu_bwd(_lib.ptr(dy2), _lib.ptr(aux), _lib.ptr(dpre), _lib.c_ll(dy2.numel()),
-                                       _lib.stream_ptr()),
+                _lib.lib().pb_gelu_bwd(_lib.addr(dy2), _lib.addr(aux), _lib.addr(dpre), dy2.numel(),
+                                       _lib.stream_addr()),
                 "pb_gelu_bwd",
             )
             dy2 = dpre
@@ -177,7 +177,7 @@ def _norm_scratch(H: int, device) -> torch.Tensor:
     key = (device.index, H)
     buf = _NORM_SCRATCH.get(key)
     if buf is None:
-        n = int(_lib.lib().pb_norm_bwd_scratch_floats(_lib.c_int(H), _lib.c_int(sm_count())))
+        n = int(_lib.lib().pb_norm_bwd_scratch_floats(H, sm_count()))
         buf = torch.empty(n, dtype=torch.float32, device=device)
         _NORM_SCRATCH[key] = buf
     return buf
@@ -210,9 +210,9 @@ class _NormFn(torch.autograd.Function):
         rstd = torch.empty(T, dtype=torch.float32, device=x.device)
         mean = torch.empty(T, dtype=torch.float32, device=x.device) if layer else None
         _lib.check(
-            _lib.lib().pb_norm_fwd(_lib.ptr(x2), _lib.ptr(weight), _lib.ptr(bias), _lib.ptr(y), _lib.ptr(mean),
-                                   _lib.ptr(rstd), _lib.c_int(T), _lib.c_int(H), _lib.c_float(eps),
-                                   _lib.c_int(int(layer)), _lib.stream_ptr()),
+            _lib.lib().pb_norm_fwd(_lib.addr(x2), _lib.addr(weight), _lib.addr(bias), _lib.addr(y), _lib.addr(mean),
+                                   _lib.addr(rstd), T, H, eps,
+                                   int(layer), _lib.stream_addr()),
             "pb_norm_fwd",
         )
         ctx.save_for_backward(x2, mean, rstd)
@@ -253,11 +253,10 @@ class _NormFn(torch.autograd.Function):
             bmg = getattr(bias, "main_grad", None)
             db = bmg if (use_main and bmg is not None) else torch.empty(H, dtype=torch.float32, device=x2.device)
         _lib.check(
-            _lib.lib().pb_norm_bwd_res(_lib.ptr(dy2), _lib.ptr(x2), _lib.ptr(weight), _lib.ptr(mean), _lib.ptr(rstd),
-                                       _lib.ptr(dres), _lib.ptr(dx), _lib.ptr(dw), _lib.ptr(db), _lib.ptr(None),
-                                       _lib.ptr(None), _lib.c_int(int(use_main)),
-                                       _lib.ptr(_norm_scratch(H, x2.device)), _lib.c_int(T), _lib.c_int(H),
-                                       _lib.c_int(int(ctx.layer)), _lib.c_int(sm_count()), _lib.stream_ptr()),
+            _lib.lib().pb_norm_bwd_res(_lib.addr(dy2), _lib.addr(x2), _lib.addr(weight), _lib.addr(mean),
+                                       _lib.addr(rstd), _lib.addr(dres), _lib.addr(dx), _lib.addr(dw), _lib.addr(db),
+                                       None, None, int(use_main), _lib.addr(_norm_scratch(H, x2.device)), T, H,
+                                       int(ctx.layer), sm_count(), _lib.stream_addr()),
             "pb_norm_bwd_res",
         )
         if not use_main:
@@ -302,8 +301,8 @@ class _SwiGLUFn(torch.autograd.Function):
             g2 = g2.contiguous()
         out = torch.empty(g2.shape[0], F2 // 2, device=gu.device, dtype=gu.dtype)
         _lib.check(
-            _lib.lib().pb_swiglu_fwd(_lib.ptr(g2), _lib.ptr(out), _lib.c_ll(g2.shape[0]), _lib.c_int(F2 // 2),
-                                     _lib.ptr(row_limit), _lib.stream_ptr()),
+            _lib.lib().pb_swiglu_fwd(_lib.addr(g2), _lib.addr(out), g2.shape[0], F2 // 2,
+                                     _lib.addr(row_limit), _lib.stream_addr()),
             "pb_swiglu_fwd",
         )
         ctx.save_for_backward(g2)
@@ -319,8 +318,8 @@ class _SwiGLUFn(torch.autograd.Function):
             d2 = d2.contiguous()
         dgu = torch.empty_like(g2)
         _lib.check(
-            _lib.lib().pb_swiglu_bwd(_lib.ptr(d2), _lib.ptr(g2), _lib.ptr(dgu), _lib.c_ll(g2.shape[0]),
-                                     _lib.c_int(g2.shape[1] // 2), _lib.ptr(ctx.row_limit), _lib.stream_ptr()),
+            _lib.lib().pb_swiglu_bwd(_lib.addr(d2), _lib.addr(g2), _lib.addr(dgu), g2.shape[0],
+                                     g2.shape[1] // 2, _lib.addr(ctx.row_limit), _lib.stream_addr()),
             "pb_swiglu_bwd",
         )
         return dgu.view(ctx.shape), None
@@ -347,9 +346,9 @@ def rope_tables(seq_len: int, head_dim: int, theta: float, device) -> Tuple[torc
 
 def _rope_inplace(buf: torch.Tensor, cos, sin, T: int, S: int, n_heads: int, D: int, sign: float) -> None:
     _lib.check(
-        _lib.lib().pb_rope(_lib.ptr(buf), _lib.ptr(cos), _lib.ptr(sin), _lib.c_ll(T), _lib.c_int(S),
-                           _lib.c_int(n_heads), _lib.c_int(D), _lib.c_ll(buf.stride(0)), _lib.c_float(sign),
-                           _lib.stream_ptr()),
+        _lib.lib().pb_rope(_lib.addr(buf), _lib.addr(cos), _lib.addr(sin), T, S,
+                           n_heads, D, buf.stride(0), sign,
+                           _lib.stream_addr()),
         "pb_rope",
     )
 
@@ -366,11 +365,11 @@ def flash_forward(q, k, v, B, S, Hq, Hkv, D, scale, causal=True):
     o = torch.empty(B * S, Hq * D, device=q.device, dtype=torch.bfloat16)
     lse = torch.empty(B, Hq, S, device=q.device, dtype=torch.float32)
     _lib.check(
-        _lib.lib().pb_flash_fwd(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(o), _lib.ptr(lse), _lib.c_int(B),
-                                _lib.c_int(S), _lib.c_int(Hq), _lib.c_int(Hkv), _lib.c_int(D),
-                                _lib.c_ll(q.stride(0)), _lib.c_ll(k.stride(0)), _lib.c_ll(v.stride(0)),
-                                _lib.c_ll(o.stride(0)), _lib.c_float(scale), _lib.c_int(int(causal)),
-                                _lib.ptr(_lib.err_word(q.device)), _lib.stream_ptr()),
+        _lib.lib().pb_flash_fwd(_lib.addr(q), _lib.addr(k), _lib.addr(v), _lib.addr(o), _lib.addr(lse), B,
+                                S, Hq, Hkv, D,
+                                q.stride(0), k.stride(0), v.stride(0),
+                                o.stride(0), scale, int(causal),
+                                _lib.err_addr(q.device), _lib.stream_addr()),
         "pb_flash_fwd",
     )
     return o, lse
@@ -386,13 +385,13 @@ def flash_backward(do, q, k, v, o, lse, B, S, Hq, Hkv, D, scale, causal=True, dq
     dv = dqkv[:, (Hq + Hkv) * D :]
     delta = torch.empty(B, Hq, S, device=q.device, dtype=torch.float32)
     _lib.check(
-        _lib.lib().pb_flash_bwd(_lib.ptr(do), _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(o), _lib.ptr(lse),
-                                _lib.ptr(delta), _lib.ptr(dq), _lib.ptr(dk), _lib.ptr(dv), _lib.c_int(B),
-                                _lib.c_int(S), _lib.c_int(Hq), _lib.c_int(Hkv), _lib.c_int(D),
-                                _lib.c_ll(q.stride(0)), _lib.c_ll(k.stride(0)), _lib.c_ll(v.stride(0)),
-                                _lib.c_ll(o.stride(0)), _lib.c_ll(do.stride(0)), _lib.c_ll(dqkv.stride(0)),
-                                _lib.c_float(scale), _lib.c_int(int(causal)), _lib.ptr(_lib.err_word(q.device)),
-                                _lib.stream_ptr()),
+        _lib.lib().pb_flash_bwd(_lib.addr(do), _lib.addr(q), _lib.addr(k), _lib.addr(v), _lib.addr(o), _lib.addr(lse),
+                                _lib.addr(delta), _lib.addr(dq), _lib.addr(dk), _lib.addr(dv), B,
+                                S, Hq, Hkv, D,
+                                q.stride(0), k.stride(0), v.stride(0),
+                                o.stride(0), do.stride(0), dqkv.stride(0),
+                                scale, int(causal), _lib.err_addr(q.device),
+                                _lib.stream_addr()),
         "pb_flash_bwd",
     )
     return dq, dk, dv, dqkv
@@ -479,9 +478,9 @@ class _CrossEntropyFn(torch.autograd.Function):
         n_valid = torch.empty((), dtype=torch.float32, device=dev) if reduction == "mean" else None
         loss = torch.empty((), dtype=torch.float32, device=dev)
         _lib.check(
-            _lib.lib().pb_xent(_lib.ptr(logits), _lib.ptr(dlogits), _lib.ptr(tgt), _lib.ptr(loss_rows),
-                               _lib.ptr(n_valid), _lib.ptr(loss), _lib.c_ll(T), _lib.c_int(vocab),
-                               _lib.c_ll(logits.stride(0)), _lib.c_ll(ignore_index), _lib.stream_ptr()),
+            _lib.lib().pb_xent(_lib.addr(logits), _lib.addr(dlogits), _lib.addr(tgt), _lib.addr(loss_rows),
+                               _lib.addr(n_valid), _lib.addr(loss), T, vocab,
+                               logits.stride(0), ignore_index, _lib.stream_addr()),
             "pb_xent",
         )
         ctx.save_for_backward(dlogits)
@@ -492,8 +491,8 @@ class _CrossEntropyFn(torch.autograd.Function):
         (dlogits,) = ctx.saved_tensors
         scale = dloss.to(torch.float32).reshape(1).contiguous()
         _lib.check(
-            _lib.lib().pb_scale_bf16(_lib.ptr(dlogits), _lib.ptr(scale), _lib.c_ll(dlogits.numel()),
-                                     _lib.stream_ptr()),
+            _lib.lib().pb_scale_bf16(_lib.addr(dlogits), _lib.addr(scale), dlogits.numel(),
+                                     _lib.stream_addr()),
             "pb_scale_bf16",
         )
         return dlogits, None, None, None, None, None
@@ -526,8 +525,8 @@ def _embed_wgrad(ids, dout, wte, wpe, S):
         pmg = getattr(wpe, "main_grad", None)
         dp = pmg if (pmg is not None and pmg.dtype == torch.float32) else torch.zeros(wpe.shape, dtype=torch.float32, device=wpe.device)
     _lib.check(
-        _lib.lib().pb_embed_bwd(_lib.ptr(ids), _lib.ptr(dout), _lib.ptr(dw), _lib.ptr(dp), _lib.c_ll(T),
-                                _lib.c_int(H), _lib.c_int(S), _lib.c_ll(wte.shape[0]), _lib.stream_ptr()),
+        _lib.lib().pb_embed_bwd(_lib.addr(ids), _lib.addr(dout), _lib.addr(dw), _lib.addr(dp), T,
+                                H, S, wte.shape[0], _lib.stream_addr()),
         "pb_embed_bwd",
     )
     if dw is not wmg:
@@ -543,8 +542,8 @@ class _EmbeddingFn(torch.autograd.Function):
         T, H = flat.numel(), wte.shape[1]
         out = torch.empty(T, H, device=wte.device, dtype=wte.dtype)
         _lib.check(
-            _lib.lib().pb_embed_fwd(_lib.ptr(flat), _lib.ptr(wte), _lib.ptr(wpe), _lib.ptr(out), _lib.c_ll(T),
-                                    _lib.c_int(H), _lib.c_int(S), _lib.c_ll(wte.shape[0]), _lib.stream_ptr()),
+            _lib.lib().pb_embed_fwd(_lib.addr(flat), _lib.addr(wte), _lib.addr(wpe), _lib.addr(out), T,
+                                    H, S, wte.shape[0], _lib.stream_addr()),
             "pb_embed_fwd",
         )
         ctx.save_for_backward(flat)

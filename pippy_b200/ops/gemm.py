@@ -73,19 +73,19 @@ def gemm(
         assert residual.shape == (M, N) and residual.stride(1) == 1 and residual.dtype == torch.bfloat16
     if aux is not None:
         assert aux.shape == (M, N) and aux.stride(0) == out.stride(0) and aux.dtype == torch.bfloat16
-    stream = _lib.stream_ptr()
-    key = (a.device.index, stream.value)
+    stream = _lib.stream_addr()
+    key = (a.device.index, stream)
     ws = _SPLIT_WS.get(key)
 
     def call(ws, ask):
         return _lib.lib().pb_gemm_bf16_ws(
-            _lib.ptr(a), _lib.ptr(b), _lib.ptr(out),
-            _lib.c_int(M), _lib.c_int(N), _lib.c_int(K),
-            _lib.c_ll(a.stride(0)), _lib.c_ll(b.stride(0)), _lib.c_ll(out.stride(0)),
-            _lib.c_int(int(a_mn)), _lib.c_int(int(b_mn)),
-            _lib.ptr(bias), _lib.ptr(residual), _lib.c_ll(residual.stride(0) if residual is not None else 0),
-            _lib.ptr(aux), _lib.c_int(act), _lib.c_int(int(out_fp32)), _lib.c_int(int(accumulate)),
-            _lib.c_int(variant), _lib.ptr(ws), _lib.c_int(ask), _lib.ptr(_lib.err_word(a.device)), stream,
+            _lib.addr(a), _lib.addr(b), _lib.addr(out),
+            M, N, K,
+            a.stride(0), b.stride(0), out.stride(0),
+            int(a_mn), int(b_mn),
+            _lib.addr(bias), _lib.addr(residual), residual.stride(0) if residual is not None else 0,
+            _lib.addr(aux), act, int(out_fp32), int(accumulate),
+            variant, _lib.addr(ws), ask, _lib.err_addr(a.device), stream,
         )
 
     rc = call(ws, 1)
@@ -107,7 +107,7 @@ def gemm(
 def set_sm_reserve(n: int) -> None:
     """Keeps ``n`` SMs out of the persistent GEMM grid so that communication kernels (NCCL point-to-point, the
     fused collectives of this package) always find a free SM while a GEMM is running."""
-    _lib.lib().pb_set_sm_reserve(_lib.c_int(int(n)))
+    _lib.lib().pb_set_sm_reserve(int(n))
 
 
 def set_tile_band(n: int) -> None:
@@ -115,4 +115,4 @@ def set_tile_band(n: int) -> None:
     inside a band (0 restores the default of 8 for CTA-pair tiles).  Which band is fastest depends on the shape by
     a few percent (measured under sustained load on the 7B shapes: 4 is 5 % ahead on the QKV forward, 8 is 2 % ahead
     on the gate/up dgrad, the rest within noise), so the default is left alone; the knob is for tuning a new shape."""
-    _lib.lib().pb_set_gemm_group_m(_lib.c_int(int(n)))
+    _lib.lib().pb_set_gemm_group_m(int(n))

@@ -91,10 +91,10 @@ class FusedAdamW:
             g.fold_autograd_grads()
             if g.data.is_cuda and g.data.dtype == torch.bfloat16 and g.grad.dtype == torch.float32:
                 rc = _lib.lib().pb_adamw(
-                    _lib.ptr(g.data), _lib.ptr(master), _lib.ptr(g.grad), _lib.ptr(m), _lib.ptr(v),
-                    _lib.c_ll(g.numel), _lib.c_float(self.lr), _lib.c_float(b1), _lib.c_float(b2),
-                    _lib.c_float(self.eps), _lib.c_float(self.weight_decay), _lib.c_int(self.step_count),
-                    _lib.c_float(grad_scale), _lib.c_int(int(zero_grad)), _lib.stream_ptr(),
+                    _lib.addr(g.data), _lib.addr(master), _lib.addr(g.grad), _lib.addr(m), _lib.addr(v),
+                    g.numel, self.lr, b1, b2,
+                    self.eps, self.weight_decay, self.step_count,
+                    grad_scale, int(zero_grad), _lib.stream_addr(),
                 )
                 _lib.check(rc, "pb_adamw")
             else:
