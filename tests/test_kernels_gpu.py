@@ -242,6 +242,43 @@ def test_linear_main_grad_accumulates_fp32():
     assert w.grad is None and _rel(w.main_grad, ref) < 1e-3
 
 
+@pytest.mark.parametrize("T,C,ld", [(1, 8, 8), (33, 264, 272), (2048, 768, 768), (1000, 2304, 2304), (257, 1024, 1028), (100, 30, 30)])
+def test_column_sums(T, C, ld):
+    """Bias gradients: whole and partial 256-column groups, fewer rows than a CTA takes, pitches that are no multiple of 8
+    (the 4-byte kernel).  fp32 sums of T bf16 values: the order changes them by T * 2^-24 of the absolute sum at most."""
+    from pippy_b200.ops import _lib
+
+    x = _bf16(T, ld)
+    out = torch.ones(C, device="cuda")
+    _lib.check(_lib.lib().pb_colsum_bf16(_lib.ptr(x), _lib.ptr(out), _lib.c_ll(T), _lib.c_int(C), _lib.c_ll(ld),
+                                         _lib.stream_ptr()), "pb_colsum_bf16")
+    ref = x[:, :C].double().sum(0) + 1
+    bound = (T + 8) * 2 ** -24 * (x[:, :C].double().abs().sum(0) + 1)
+    assert ((out.double() - ref).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("T", [1, 31, 33, 257, 3000])
+@pytest.mark.parametrize("layer", [False, True])
+def test_norm_weight_gradient_fold(T, layer):
+    """From one partial row to a full grid of them, against fp64; the bias has its own half of the fold."""
+    from pippy_b200.ops import functional as pf
+
+    H = 776
+    x = _bf16(T, H).requires_grad_()
+    w, b = torch.nn.Parameter(_bf16(H)), torch.nn.Parameter(_bf16(H))
+    w.main_grad, b.main_grad = (torch.randn(H, device="cuda") for _ in range(2))
+    w0, b0 = w.main_grad.double(), b.main_grad.double()
+    dy = _bf16(T, H)
+    (pf.layer_norm(x, w, b) if layer else pf.rms_norm(x, w)).backward(dy)
+    xd = x.detach().double()
+    mean = xd.mean(-1, keepdim=True) if layer else 0.0
+    xh = (xd - mean) * torch.rsqrt((xd - mean).pow(2).mean(-1, keepdim=True) + 1e-5)
+    terms = dy.double() * xh
+    assert ((w.main_grad.double() - w0 - terms.sum(0)).abs() <= 1e-5 * (terms.abs().sum(0) + 1)).all()
+    if layer:
+        assert ((b.main_grad.double() - b0 - dy.double().sum(0)).abs() <= 1e-5 * (dy.double().abs().sum(0) + 1)).all()
+
+
 def test_cross_entropy():
     from pippy_b200.ops import functional as pf
 
