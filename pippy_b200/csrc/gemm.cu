@@ -351,10 +351,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             m0 -= chunk * p.chunk_rows;  // own shard, read in place
           } else {
             tma_a = &tmA2;
-            if (!pbp::wait_flag_gpu(p.tile_flags + tm, p.epoch, p.err, ERR_PEER_TIMEOUT)) {
-              ok = false;
-              break;
-            }
+            // the verdict is the warp's: lanes that went different ways would wait for one another below
+            ok = __all_sync(0xffffffffu, pbp::wait_flag_gpu(p.tile_flags + tm, p.epoch, p.err, ERR_PEER_TIMEOUT));
+            if (!ok) break;
             asm volatile("fence.proxy.async.global;" ::: "memory");  // copied rows -> visible to the TMA engine
           }
         }
