@@ -67,13 +67,10 @@ class GPT2Block(nn.Module):
 
     def forward(self, x, B: int, S: int):
         cfg = self.cfg
-        # norm.fork: the residual branch's gradient is added inside the norm-backward kernel
-        n, x = self.ln_1.fork(x)
-        qkv = self.attn_c_attn(n)
+        qkv = self.attn_c_attn(self.ln_1(x))
         att = pf.rope_attention(qkv, None, None, B, S, cfg.n_heads, cfg.n_heads, cfg.head_dim)
         x = self.attn_c_proj(att, residual=x)
-        n, x = self.ln_2.fork(x)
-        h = self.mlp_c_fc(n, activation="gelu_tanh")
+        h = self.mlp_c_fc(self.ln_2(x), activation="gelu_tanh")
         return self.mlp_c_proj(h, residual=x)
 
 

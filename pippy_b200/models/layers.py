@@ -59,10 +59,6 @@ class LayerNorm(nn.Module):
     def forward(self, x):
         return pf.layer_norm(x, self.weight, self.bias, self.eps)
 
-    def fork(self, x):
-        """``(norm(x), x)``; pass the second result to the residual add (see ``pf.rms_norm_fork``)."""
-        return pf.layer_norm_fork(x, self.weight, self.bias, self.eps)
-
 
 class Embedding(nn.Module):
     """Token embedding with an optional learned position table; returns ``[B*S, H]``."""

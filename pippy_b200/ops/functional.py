@@ -283,13 +283,6 @@ def rms_norm(x, weight, eps: float = 1e-5):
     return (y * weight.float()).to(x.dtype)
 
 
-def layer_norm_fork(x, weight, bias, eps: float = 1e-5):
-    """``(layer_norm(x), x)``: as :func:`rms_norm_fork`."""
-    if _use_kernels(x):
-        return _NormFn.apply(x, weight, bias, eps, True, True)
-    return layer_norm(x, weight, bias, eps), x
-
-
 def layer_norm(x, weight, bias, eps: float = 1e-5):
     if _use_kernels(x):
         return _NormFn.apply(x, weight, bias, eps, True, False)
