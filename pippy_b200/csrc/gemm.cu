@@ -15,6 +15,7 @@
 #include "tc05.cuh"
 #include "peer.cuh"
 
+#include <atomic>
 #include <string.h>
 
 extern "C" void pb_count_launch(int n);
@@ -77,10 +78,12 @@ struct GemmParams {
   // ---- split contraction (plain GEMMs): tiles from `dp_tiles` on are cut into `splits` ranges of k-blocks, one work
   // item each.  Every item leaves its fp32 partial tile in `split_ws`; the one that arrives last at the tile's counter
   // (per 32 rows) adds the partials in range order, so the result does not depend on which one that was, and runs
-  // the epilogue.  Nobody waits.  The counters are zero before and after every launch.
+  // the epilogue.  Nobody waits.  A counter holds the launch's tag | arrivals (low 4 bits); under any other tag it counts
+  // as zero, so that what a launch that gave up left behind means nothing to the next one.
   int dp_tiles, splits;
   float* split_ws;
-  int* split_counters;
+  unsigned long long* split_counters;
+  unsigned long long split_tag;
 };
 
 constexpr int MAX_GROUPS = 8;
@@ -559,6 +562,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         finish = false;
         if (row_w < m_limit) {
           float4* own = reinterpret_cast<float4*>(p.split_ws + (first_item + range) * ITEM + slot);
+          unsigned long long* counter =
+              p.split_counters + (first_item / p.splits) * (4 * kCtaGroup) + cta_rank * 4 + quarter;
+          unsigned long long seen = 0;
+          if (lane == 0) seen = __ldcg(counter);  // a guess for the exchange below, there by the time it is needed
 #pragma unroll 1
           for (int c = 0; c < BN / 32 && n0 + c * 32 < p.N; ++c) {
             uint32_t r[32];
@@ -573,14 +580,20 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           __threadfence();
           __syncwarp();
           int arrived = 0;
-          int* counter = p.split_counters + (first_item / p.splits) * (4 * kCtaGroup) + cta_rank * 4 + quarter;
-          if (lane == 0) arrived = atomicAdd(counter, 1);
+          if (lane == 0) {
+            for (int attempt = 0; attempt < 16; ++attempt) {  // fails only when another of the <= 8 ranges got in first
+              const unsigned long long base = (seen & ~15ull) == p.split_tag ? seen : p.split_tag;
+              const unsigned long long old = atomicCAS(counter, seen, base + 1);
+              if (old == seen) {
+                arrived = (int)(base & 15ull);
+                break;
+              }
+              seen = old;
+            }
+          }
           arrived = __shfl_sync(0xffffffffu, arrived, 0);
           finish = arrived == p.splits - 1;
-          if (finish) {
-            __threadfence();
-            if (lane == 0) *counter = 0;  // as the next launch expects it
-          }
+          if (finish) __threadfence();
         }
       }
       if (!finish) {
@@ -1029,6 +1042,7 @@ struct GemmPlan {
 
 constexpr long long SPLIT_ITEM_BYTES = 128 * 256 * 4;  // partial of one CTA, largest variant
 constexpr int SPLIT_COUNTERS = 1024;                   // 4 per CTA of a split tile, at most 148 CTAs
+std::atomic<unsigned long long> g_split_calls{0};      // source of the launches' tags (never 0: cleared counters)
 
 // Estimated SM cycles of `variant` and the best split of its last wave.  Tiles run in waves of one per worker (CTA or
 // CTA pair).  When r tiles are left for the last wave they are cut into s ranges of k-blocks, r * s <= workers: the
@@ -1089,12 +1103,13 @@ void pb_set_gemm_group_m(int n) { pb::g_group_m = n < 0 ? 0 : n; }
 // variant: 0 = automatic, 1 = single-CTA tiles (128 x 256), 2 = CTA-pair tiles (256 x 256),
 //          3 = single-CTA 128 x 128.
 // Returns 0 on success, a negative value for an argument error, a positive CUDA error otherwise.
-// `split_ws`: pb_gemm_split_ws_bytes() bytes that no other stream uses, its last 4 KB (the counters) zero before the
-// first call and left zero by every call; null = the contraction is never split.  With `ask_ws` != 0 the call returns
+// `split_ws`: pb_gemm_split_ws_bytes() bytes that no other stream uses, its last 8 KB (the counters) cleared before the
+// first call; null = the contraction is never split.  A call under capture bakes its tag into the graph, which therefore
+// has to clear the counters itself before the kernel.  With `ask_ws` != 0 the call returns
 // PB_GEMM_WANTS_WS, without launching anything, where a split needs a workspace and none is given, or the given one
 // (which outlives the call) would become part of a graph under capture.
 #define PB_GEMM_WANTS_WS (-100)
-long long pb_gemm_split_ws_bytes() { return 148LL * SPLIT_ITEM_BYTES + SPLIT_COUNTERS * 4; }
+long long pb_gemm_split_ws_bytes() { return 148LL * SPLIT_ITEM_BYTES + SPLIT_COUNTERS * 8; }
 
 // out: variant, whole tiles, ranges per split tile, split work items
 void pb_gemm_plan(int M, int N, int K, int sms, int may_split, int* out) {
@@ -1167,7 +1182,11 @@ int pb_gemm_bf16_ws(const void* A, const void* B, void* C, int M, int N, int K, 
   p.dp_tiles = plan.dp_tiles;
   p.splits = plan.splits;
   p.split_ws = reinterpret_cast<float*>(split_ws);
-  p.split_counters = reinterpret_cast<int*>(reinterpret_cast<char*>(split_ws) + 148LL * SPLIT_ITEM_BYTES);
+  if (plan.splits > 1) {
+    p.split_counters =
+        reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(split_ws) + 148LL * SPLIT_ITEM_BYTES);
+    p.split_tag = (g_split_calls.fetch_add(1, std::memory_order_relaxed) + 1) << 4;
+  }
   switch (variant) {
     case 1: return launch_gemm<1, 256, 4>(tmA, tmB, p, sms, stream);
     case 2: return launch_gemm<2, 256, 6>(tmA, tmB, p, sms, stream);

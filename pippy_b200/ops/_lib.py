@@ -15,7 +15,6 @@ import torch
 _LIB = None
 _LOCK = threading.Lock()
 _ERR_WORDS: dict[int, torch.Tensor] = {}
-ON_DEVICE_ERROR: list = []  # called when check_device_errors finds an error, before it raises
 
 _LIB_DIR = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "lib")
 # PIPPY_BOUNDS_CHECK=1 selects the debug library, whose kernels validate the indices they read from tensors
@@ -133,8 +132,6 @@ def check_device_errors() -> None:
         code = int(w.item())
         if code != 0:
             w.zero_()
-            for fn in ON_DEVICE_ERROR:
-                fn()
             raise KernelError(f"device {idx}: kernel error code {code} (1 = bounded wait ran out, 3 = peer wait ran out, "
                               "4 = MoE receive buffer overflow, 5 = index out of range in a bounds-checking build)")
 

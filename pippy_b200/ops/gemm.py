@@ -12,15 +12,14 @@ ACT_GELU_TANH = 1
 
 
 # Workspaces of the split contraction (partial tiles + arrival counters), one per device and stream: calls on a stream
-# run one after the other, and every call leaves the counters at zero for the next.  At most _MAX_SPLIT_WS are kept;
-# the allocator frees a dropped one in the order of the stream that used it.  A capture gets a workspace of its own,
-# which lives in the graph's pool and is cleared by the graph: a replay may run beside eager calls on the stream it was
-# captured on.
+# run one after the other, and each tells its own arrivals from whatever an earlier one left in the counters.  At most
+# _MAX_SPLIT_WS are kept; the allocator frees a dropped one in the order of the stream that used it.  A capture gets a
+# workspace of its own, which lives in the graph's pool and whose counters the graph clears at every replay (they all
+# carry the same tag): a replay may run beside eager calls on the stream it was captured on.
 _SPLIT_WS: "OrderedDict[tuple, torch.Tensor]" = OrderedDict()
 _MAX_SPLIT_WS = 8
 _WANTS_WS = -100
-_COUNTER_BYTES = 4096
-_lib.ON_DEVICE_ERROR.append(_SPLIT_WS.clear)  # a call that gave up may have left its counters behind
+_COUNTER_BYTES = 8192
 
 
 def _new_split_ws(device: torch.device) -> torch.Tensor:

@@ -115,6 +115,24 @@ def test_gemm_split_contraction(M, N, K):
         assert torch.equal(captured, out)
 
 
+@pytest.mark.parametrize("M,N,K", [(77, 4096, 4096), (2048, 768, 16384)])
+def test_gemm_split_ignores_leftover_counters(M, N, K):
+    """Whatever a launch that gave up left in the arrival counters of the kept workspace, the next call is right."""
+    from pippy_b200.ops import _lib
+    from pippy_b200.ops import gemm as mod
+
+    a, b = _bf16(M, K), _bf16(K, N)
+    out = mod.gemm(a, b, b_mn=True)
+    ws = mod._SPLIT_WS[(a.device.index, _lib.stream_addr())]
+    counters = ws[-mod._COUNTER_BYTES:].view(torch.int64)
+    used = counters.clone()
+    assert used.any()
+    for left in (torch.ones_like(used), used, used - 1, torch.randint(-2 ** 62, 2 ** 62, used.shape, device="cuda")):
+        counters.copy_(left)
+        for _ in range(2):
+            assert torch.equal(mod.gemm(a, b, b_mn=True), out)
+
+
 @pytest.mark.parametrize("H", [768, 4096, 5120])
 @pytest.mark.parametrize("layer", [False, True])
 def test_norm(H, layer):
