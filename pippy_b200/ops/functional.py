@@ -170,17 +170,11 @@ def linear(x, weight, bias=None, residual=None, activation: Optional[str] = None
 # ------------------------------------------------------------------------------------------------
 # normalisation
 # ------------------------------------------------------------------------------------------------
-_NORM_SCRATCH = {}
-
-
 def _norm_scratch(H: int, device) -> torch.Tensor:
-    key = (device.index, H)
-    buf = _NORM_SCRATCH.get(key)
-    if buf is None:
-        n = int(_lib.lib().pb_norm_bwd_scratch_floats(H, sm_count()))
-        buf = torch.empty(n, dtype=torch.float32, device=device)
-        _NORM_SCRATCH[key] = buf
-    return buf
+    """Partial sums that the norm backward's two kernels hand over: each call's own, since another stream, a captured
+    graph or another thread may be between the same two kernels."""
+    n = int(_lib.lib().pb_norm_bwd_scratch_floats(H, sm_count()))
+    return torch.empty(n, dtype=torch.float32, device=device)
 
 
 _lib_scratch_restype_set = False
@@ -252,10 +246,11 @@ class _NormFn(torch.autograd.Function):
         if ctx.layer:
             bmg = getattr(bias, "main_grad", None)
             db = bmg if (use_main and bmg is not None) else torch.empty(H, dtype=torch.float32, device=x2.device)
+        scratch = _norm_scratch(H, x2.device)
         _lib.check(
             _lib.lib().pb_norm_bwd_res(_lib.addr(dy2), _lib.addr(x2), _lib.addr(weight), _lib.addr(mean),
                                        _lib.addr(rstd), _lib.addr(dres), _lib.addr(dx), _lib.addr(dw), _lib.addr(db),
-                                       None, None, int(use_main), _lib.addr(_norm_scratch(H, x2.device)), T, H,
+                                       None, None, int(use_main), _lib.addr(scratch), T, H,
                                        int(ctx.layer), sm_count(), _lib.stream_addr()),
             "pb_norm_bwd_res",
         )

@@ -297,6 +297,41 @@ def test_norm_weight_gradient_fold(T, layer):
         assert ((b.main_grad.double() - b0 - dy.double().sum(0)).abs() <= 1e-5 * (dy.double().abs().sum(0) + 1)).all()
 
 
+def test_norm_backward_beside_other_streams_and_replays():
+    """Weight gradients of the same width from two streams at once, and from a captured backward that is replayed beside
+    eager ones: each has its own partial sums."""
+    from pippy_b200.ops import functional as pf
+
+    T, H = 2048, 1024
+    x, dy = [_bf16(T, H).requires_grad_() for _ in range(2)], [_bf16(T, H) for _ in range(2)]
+    ws = [torch.nn.Parameter(_bf16(H)) for _ in range(2)]
+    for w in ws:
+        w.main_grad = torch.zeros(H, device="cuda")
+
+    def backward(i):
+        return torch.autograd.grad(pf.rms_norm(x[i], ws[i]), x[i], dy[i])[0]
+
+    refs = []
+    for i in range(2):
+        backward(i)
+        refs.append(ws[i].main_grad.clone())
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=streams[0]):
+        ws[0].main_grad.zero_()
+        backward(0)
+    for first in (lambda: (ws[0].main_grad.zero_(), backward(0)), graph.replay):
+        for _ in range(20):
+            with torch.cuda.stream(streams[0]):
+                first()
+            with torch.cuda.stream(streams[1]):
+                ws[1].main_grad.zero_()
+                backward(1)
+            torch.cuda.synchronize()
+            assert torch.equal(ws[0].main_grad, refs[0]) and torch.equal(ws[1].main_grad, refs[1])
+
+
 def test_cross_entropy():
     from pippy_b200.ops import functional as pf
 
