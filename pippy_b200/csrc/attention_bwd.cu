@@ -17,6 +17,7 @@
 // eight warps take the even and the odd blocks: each group owns one TMEM score buffer and one P/dS buffer, the
 // groups drift apart in phase, and every scheduler has four warps to switch between.
 // A small pre-pass computes delta = rowsum(dO * O).
+#include "launch.cuh"
 #include "tc05.cuh"
 
 #include <math_constants.h>
@@ -521,13 +522,8 @@ static int launch_bwd(const CUtensorMap& x1, const CUtensorMap& x2, const CUtens
                       BwdParams p, cudaStream_t stream) {
   constexpr int NCH = D / 64;
   constexpr int SMEM = 2 * NCH * 128 * 128 + 2 * NST * NCH * 64 * 128 + 2048 + 256;
-  auto kern = fa_bwd_kernel<D, kMode>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  constexpr auto kern = fa_bwd_kernel<D, kMode>;
+  if (cudaError_t e = pb::allow_smem<kern, SMEM>(); e != cudaSuccess) return (int)e;
   const int tiles = (p.S + BR - 1) / BR, heads = (kMode == 0 ? p.Hkv : p.Hq) * p.B;
   p.head_group = attention_head_group(tiles, heads);
   const unsigned grid = (unsigned)tiles * heads;

@@ -12,6 +12,7 @@
 // Warp roles: 0 = TMA producer, 1 = MMA issuer (+TMEM owner), 2..9 = softmax/epilogue: two warps per TMEM lane
 // quarter, each owning 64 of the block's 128 columns (row maxima are exchanged through shared memory), so every
 // scheduler has two warps to alternate between.
+#include "launch.cuh"
 #include "tc05.cuh"
 
 #include <math_constants.h>
@@ -604,13 +605,8 @@ static int launch_fwd2(const CUtensorMap& tq, const CUtensorMap& tk, const CUten
                        cudaStream_t stream) {
   constexpr int TILE = (D / 64) * 128 * 128;
   constexpr int SMEM = 6 * TILE + 256;
-  auto kern = fa_fwd2_kernel<D>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  constexpr auto kern = fa_fwd2_kernel<D>;
+  if (cudaError_t e = pb::allow_smem<kern, SMEM>(); e != cudaSuccess) return (int)e;
   const int tiles = (p.S + 2 * BM - 1) / (2 * BM);
   p.head_group = attention_head_group(tiles, p.Hq * p.B);
   kern<<<(unsigned)tiles * p.Hq * p.B, 320, SMEM, stream>>>(tq, tk, tv, p);
@@ -623,13 +619,8 @@ static int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
                       cudaStream_t stream) {
   constexpr int TILE = (D / 64) * 128 * 128;
   constexpr int SMEM = 5 * TILE + 2048 + 256;
-  auto kern = fa_fwd_kernel<D>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  constexpr auto kern = fa_fwd_kernel<D>;
+  if (cudaError_t e = pb::allow_smem<kern, SMEM>(); e != cudaSuccess) return (int)e;
   const unsigned grid = (unsigned)((p.S + BM - 1) / BM) * p.Hq * p.B;
   kern<<<grid, 320, SMEM, stream>>>(tq, tk, tv, p);
   pb_count_launch(1);

@@ -12,6 +12,7 @@
 //
 // kCtaGroup == 2 pairs two CTAs of a cluster on one 256 x BN tile (tcgen05 cta_group::2): each
 // CTA loads its own 128 rows of A and its own half of B; the leader CTA issues the MMAs.
+#include "launch.cuh"
 #include "tc05.cuh"
 #include "peer.cuh"
 
@@ -984,13 +985,8 @@ static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParam
   constexpr int A_BYTES = BM_CTA * BK * 2;
   constexpr int B_BYTES = (BN / kCtaGroup) * BK * 2;
   constexpr int SMEM = kStages * (A_BYTES + B_BYTES) + 1024 + 256 + 4 * 32 * 144;
-  auto kern = gemm_bf16_kernel<kCtaGroup, BN, kStages>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  constexpr auto kern = gemm_bf16_kernel<kCtaGroup, BN, kStages>;
+  if (cudaError_t e = pb::allow_smem<kern, SMEM>(); e != cudaSuccess) return (int)e;
   const int tile_m = BM_CTA * kCtaGroup;
   p.num_m_tiles = (p.M + tile_m - 1) / tile_m;
   p.num_n_tiles = (p.N + BN - 1) / BN;

@@ -8,6 +8,7 @@
 #include <stdint.h>
 
 #include "dbgcheck.cuh"
+#include "launch.cuh"
 
 extern "C" void pb_count_launch(int n);
 
@@ -271,13 +272,7 @@ int pb_xent(const void* logits, void* dlogits, const long long* targets, float* 
     xent_row_kernel<128><<<(unsigned)T, 128, smem, stream>>>(L, D, targets, loss_rows, n_valid, V, ld,
                                                              ignore_index PB_DBG_ARGS(V));
   } else if (V <= ROW_WIDE) {
-    static bool attr_set = false;
-    if (!attr_set) {
-      cudaError_t e = cudaFuncSetAttribute(xent_row_kernel<THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           ROW_WIDE * 2);
-      if (e != cudaSuccess) return (int)e;
-      attr_set = true;
-    }
+    if (cudaError_t e = pb::allow_smem<xent_row_kernel<THREADS>, ROW_WIDE * 2>(); e != cudaSuccess) return (int)e;
     xent_row_kernel<THREADS><<<(unsigned)T, THREADS, smem, stream>>>(L, D, targets, loss_rows, n_valid, V, ld,
                                                                      ignore_index PB_DBG_ARGS(V));
   } else {
