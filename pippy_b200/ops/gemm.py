@@ -89,8 +89,11 @@ def gemm(
 
     rc = call(ws, 1)
     if rc == _WANTS_WS:  # none kept for this stream, or the stream is being captured
-        ws = _new_split_ws(a.device)
-        if not torch.cuda.is_current_stream_capturing():
+        try:
+            ws = _new_split_ws(a.device)
+        except torch.OutOfMemoryError:
+            ws = None  # the same call without a split needs no workspace
+        if ws is not None and not torch.cuda.is_current_stream_capturing():
             _SPLIT_WS[key] = ws
             while len(_SPLIT_WS) > _MAX_SPLIT_WS:
                 _SPLIT_WS.popitem(last=False)

@@ -133,6 +133,23 @@ def test_gemm_split_ignores_leftover_counters(M, N, K):
             assert torch.equal(mod.gemm(a, b, b_mn=True), out)
 
 
+def test_gemm_without_memory_for_a_split(monkeypatch):
+    """A call whose workspace cannot be allocated runs unsplit, keeps nothing, and the next one tries again."""
+    from pippy_b200.ops import gemm as mod
+
+    def refuse(device):
+        raise torch.OutOfMemoryError("no memory left")
+
+    a, b = _bf16(77, 4096), _bf16(4096, 4096)
+    split = mod.gemm(a, b, b_mn=True)
+    monkeypatch.setattr(mod, "_SPLIT_WS", type(mod._SPLIT_WS)())
+    with monkeypatch.context() as m:
+        m.setattr(mod, "_new_split_ws", refuse)
+        whole = mod.gemm(a, b, b_mn=True)
+        assert _rel(whole, a.float() @ b.float()) < 1e-2 and not mod._SPLIT_WS
+    assert torch.equal(mod.gemm(a, b, b_mn=True), split) and len(mod._SPLIT_WS) == 1
+
+
 @pytest.mark.parametrize("H", [768, 4096, 5120])
 @pytest.mark.parametrize("layer", [False, True])
 def test_norm(H, layer):
