@@ -540,11 +540,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         else if (res_bf16)
           prefetch_l2(p.residual + (long long)row * p.ldr + n0, fast_chunks * 64);
       }
-      if (!mbar_wait(&tfull[acc], acc_phase, abort_flag)) {
-        ok = false;
-        break;
-      }
-      __syncwarp();
+      // the verdict is the warp's: a lane that left alone would keep the others at the exchanges below for good
+      ok = __all_sync(0xffffffffu, mbar_wait(&tfull[acc], acc_phase, abort_flag));
+      if (!ok) break;
       tc_fence_after_sync();
       const uint32_t t_row = tmem_base + acc * BN + (static_cast<uint32_t>(quarter * 32) << 16);
       int c_done = 0;
