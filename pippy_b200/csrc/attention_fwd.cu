@@ -230,7 +230,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
       }
       // combine with the other half of the row
       s_xchg[(s * 2 + half) * 128 + r] = mx;
-      got = !named_bar_or(1, 256, !got);
+      got = !named_bar_or(1, 256, !(got && ok));
       if (!got) { ok = false; break; }
       mx = fmaxf(mx, s_xchg[(s * 2 + (half ^ 1)) * 128 + r]);
       const float m_cand = fmaxf(m, mx * p.scale_log2);
@@ -240,8 +240,8 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         const float m_use = (m_cand == -CUDART_INF_F) ? 0.f : m_cand;
         const float alpha = exp2f(m - m_use);  // 0 on the first block (m = -inf)
         if (j > 0) {
-          if (!mbar_wait(&o_full[(j - 1) & 1], ((j - 1) >> 1) & 1, abort_flag)) { ok = false; break; }
-          __syncwarp();
+          // a warp whose wait ran out stays in step (the others count on it at the barriers) and says so at the next one
+          ok = __all_sync(0xffffffffu, mbar_wait(&o_full[(j - 1) & 1], ((j - 1) >> 1) & 1, abort_flag));
           tc_fence_after_sync();
 #pragma unroll
           for (int cc = 0; cc < D / 64; ++cc) {
