@@ -176,16 +176,18 @@ __global__ void __launch_bounds__(THREADS) xent_fwd_bwd_kernel(const __nv_bfloat
 #pragma unroll
     for (int j = 1; j < 8; ++j) cm = fmaxf(cm, v[j]);
     const float nm = fmaxf(m, cm);
+    const float base = nm == -CUDART_INF_F ? 0.f : nm;  // nothing but masked columns so far: they add 0, not NaN
     float add = 0.f;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) add += __expf(v[j] - nm);
-    s = s * __expf(m - nm) + add;
+    for (int j = 0; j < 8; ++j) add += __expf(v[j] - base);
+    s = s * __expf(m - base) + add;
     m = nm;
   }
   for (int c = nvec * 8 + threadIdx.x; c < V; c += THREADS) {  // ragged tail
     const float v = __bfloat162float(lr[c]);
     const float nm = fmaxf(m, v);
-    s = s * __expf(m - nm) + __expf(v - nm);
+    const float base = nm == -CUDART_INF_F ? 0.f : nm;
+    s = s * __expf(m - base) + __expf(v - base);
     m = nm;
   }
   // block combine of (m, s)

@@ -399,6 +399,41 @@ def test_cross_entropy_class_counts(V, pad, reduction):
         assert ((logits[:, :V].double() - lf.grad).abs() <= (2 ** -8 + 1e-4) * lf.grad.abs() + 1e-9).all()
 
 
+@pytest.mark.parametrize("V", [1000, 32000, 60000])
+def test_cross_entropy_infinite_and_nan_logits(V):
+    """Masked classes (-inf, among them whole vectors at the start and a lone finite class), the type's lowest value, +inf
+    and NaN in all three kernels, against 64 bits."""
+    from pippy_b200.ops import functional as pf
+
+    T, inf = 8, float("inf")
+    logits = _bf16(T, V, scale=3.0)
+    tgt = torch.randint(40, V, (T,), device="cuda")
+    logits[0, :32] = -inf
+    logits[1, :] = -inf
+    logits[1, tgt[1]] = 2.0
+    logits[2, 100:] = torch.finfo(torch.bfloat16).min
+    tgt[2] = 50
+    logits[3, tgt[3]] = -inf  # the loss is infinite, the gradient is not
+    logits[4, 7] = inf
+    logits[5, 9] = float("nan")
+    logits[6, :] = -inf
+    logits[7, ::2] = -inf
+    tgt[7] = 41
+    lf = logits.double().requires_grad_()
+    rows = F.cross_entropy(lf, tgt, reduction="none")
+    for i in range(T):
+        x = logits[i : i + 1].clone().requires_grad_()
+        loss = pf.cross_entropy(x, tgt[i : i + 1], reduction="sum")
+        loss.backward()
+        (grad,) = torch.autograd.grad(rows[i], lf, retain_graph=True)
+        if rows[i].isnan():
+            assert loss.isnan() and x.grad.isnan().any(), i
+            continue
+        assert loss.item() == rows[i].item() or abs(loss.item() - rows[i].item()) <= 1e-5 * abs(rows[i].item()) + 1e-5, i
+        # one rounding to bf16 and 1e-4 for fp32 exponentials
+        assert ((x.grad[0].double() - grad[i]).abs() <= (2 ** -8 + 1e-4) * grad[i].abs() + 1e-9).all(), i
+
+
 def test_embedding():
     from pippy_b200.ops import functional as pf
 
