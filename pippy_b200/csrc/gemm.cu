@@ -416,7 +416,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     // Under `lane == 0` issuing set the pace: a 64-deep k-block took 512 to 570 cycles with every tile shape, although
     // its four MMAs run in 256 (128 x 128 tiles).  Elected in both issuing warps, of this kernel on a B200:
     // 4096 x 4096 x 8192 weight gradient 235 -> 224 us, 8192 x 4096 x 4096 207 -> 201 us, 77 x 4096 x 4096 26.4 -> 23.7 us;
-    // a k-block takes 407 to 505 cycles, about what its operands take to arrive.
+    // a pair's k-block takes 518 cycles from the first operands to the accumulator of an 8192 x 4096 x 4096 tile, where its
+    // 128 x 256 per CTA need 512 at the tensor rate.
     if (leader) {
       const uint32_t idesc = make_idesc_bf16(BM_CTA * kCtaGroup, BN, p.a_mn, p.b_mn);
       // K-major: 16 k-elements = 32 B inside the swizzled row; MN-major: 16 k-rows of 128 B
@@ -1043,7 +1044,9 @@ std::atomic<unsigned long long> g_split_calls{0};      // source of the launches
 // wave takes 1/s of the time, plus the partial tiles' way through L2.
 //
 // Constants measured on a B200.  A 64-deep k-block takes about 480 cycles with 128 x 128 tiles, 640 with 128 x 256, 500
-// with pairs (what the operands take to arrive).  Start, first operands, last MMAs and the last tile's epilogue add
+// with pairs (2 % below their tensor rate of 512, which long main loops run at).  The epilogue is charged once, as that of a
+// plain bf16 output: one of an fp32 read-modify-write pair tile takes 9 000 to 14 000 cycles, and the waves of such a
+// weight gradient with K below about 1 200 to 1 800 are bound by it, which the rule does not see.  Start, first operands, last MMAs and the last tile's epilogue add
 // 7 000, 9 500 and 14 000.  Splitting costs 6 000 + 2 000 s with 128 x 128 tiles and 9 000 + 5 000 s with 256 columns.
 // Against the best unsplit variant, us: 77 x 4096 x 11008 46.1 -> 25.2 (s = 4), 77 x 4096 x 4096 20.6 -> 16.3 (4),
 // 2048 x 768 x 50304 192 -> 118 (3), 2999 x 5120 x 13824 321 -> 291 (4), 4096 x 4096 x 8192 205 -> 192 (2); on the other
@@ -1132,10 +1135,9 @@ int pb_gemm_bf16_ws(const void* A, const void* B, void* C, int M, int N, int K, 
   }
   int sms = sm_count - g_sm_reserve;
   if (sms < 2) sms = 2;
-  if (sms > 148) sms = 148;  // what the workspace is sized for
   GemmPlan plan{variant, 0, 1, 0, 0.0};
   if (variant == 0) {
-    plan = plan_gemm(M, N, K, sms, split_ws != nullptr || ask_ws);
+    plan = plan_gemm(M, N, K, sms, (split_ws != nullptr || ask_ws) && sms <= 148);  // the workspace is sized for 148
     if (plan.splits > 1 && ask_ws) {
       cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
       cudaError_t e = split_ws ? cudaStreamIsCapturing(stream, &capture) : cudaSuccess;
@@ -1187,13 +1189,6 @@ int pb_gemm_bf16_ws(const void* A, const void* B, void* C, int M, int N, int K, 
     case 3: return launch_gemm<1, 128, 6>(tmA, tmB, p, sms, stream);
     default: return -5;
   }
-}
-
-int pb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
-                 long long ldc, int a_mn, int b_mn, const void* bias, const void* residual, long long ldr, void* aux,
-                 int act, int out_fp32, int accumulate, int variant, int* err_dev, void* stream_) {
-  return pb_gemm_bf16_ws(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, bias, residual, ldr, aux, act, out_fp32,
-                         accumulate, variant, nullptr, 0, err_dev, stream_);
 }
 
 // Grouped GEMMs of a mixture-of-experts layer: ONE launch covers all local experts, and the group sizes stay on the

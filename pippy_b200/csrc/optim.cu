@@ -85,9 +85,10 @@ int pb_adamw(void* p, float* master, float* g, float* m, float* v, long long n, 
   a.bias_c2 = 1.f - powf(beta2, (float)step);
   a.grad_scale = grad_scale;
   long long gsz = (n / 4 + 255) / 256;
-  // Bound by HBM.  32 blocks per SM over the launch (four waves) against 16, us on one B200 (4.5 TB/s of traffic):
-  // 962 M parameters 6 003 -> 5 694, 667 M 4 165 -> 3 950, 124 M with master weights 824 -> 819; one block per 256
-  // vectors, without a cap, 4 079 at 667 M.
+  // Bound by HBM.  32 blocks per SM over the launch (four waves) against 16, us, gradients cleared in the same pass, on a
+  // B200 that reached 4.5 TB/s: 962 M parameters 6 003 -> 5 694, 667 M 4 165 -> 3 950, 124 M with master weights 824 -> 819;
+  // one block per 256 vectors, without a cap, 4 079 at 667 M.  On one that reaches 6.4 TB/s the 124 M case takes 592 and
+  // 584, no more than repeated runs differ.
   if (gsz > 148 * 32) gsz = 148 * 32;
   if (gsz < 1) gsz = 1;
   adamw_kernel<<<(unsigned)gsz, 256, 0, stream>>>(reinterpret_cast<__nv_bfloat16*>(p), master, g, m, v, n, a,
